@@ -398,7 +398,7 @@ __device__ __forceinline__ void vadv_column(const S* __restrict__ stage, const S
     C scur = ld<C, S>(stage + o + sk);
     C dup = A::sub(scur, sprev);  // stage[k+1] - stage[k]
     C bcol = A::sub(dtr, cs);
-    C corr = A::mul(-cs, dup);
+    C corr = A::mul(A::neg(cs), dup);
     C dv = A::add(A::add(A::add(A::mul(dtr, ld<C, S>(pos + o)), ld<C, S>(tens + o)), ldc<C, S>(tensstage + o)), corr);
     C cp = A::div(cs, bcol);
     C dp = A::div(dv, bcol);
@@ -424,19 +424,19 @@ __device__ __forceinline__ void vadv_column(const S* __restrict__ stage, const S
         for (int u = 0; u < D; ++u) {
             const int k = kb + u;
             if (k >= nk - 1) break;                      // uniform: every thread has the same nk
-            const C as_ = A::template scale2<-1>(-gcv);  // gav * bet_m == acol, gav = -gcv(k-1)
+            const C csp = cs;  // cs(k-1) = -acol(k): acol = gav * bet_m, gav = -gcv(k-1)
             gcv = A::template scale2<-2>(A::add(rw1[u], rw0[u]));
             cs = A::template scale2<-1>(gcv);
             const C snext = rst[u];
             const C ddown = A::neg_diff(dup, scur, sprev);  // stage[k-1] - stage[k]
             dup = A::sub(snext, scur);                     // stage[k+1] - stage[k]
-            bcol = A::sub(A::sub(dtr, as_), cs);
-            corr = A::sub(A::mul(-as_, ddown), A::mul(cs, dup));
+            bcol = A::sub(A::add(dtr, csp), cs);
+            corr = A::sub(A::mul(csp, ddown), A::mul(cs, dup));
             dv = A::add(A::add(A::add(A::mul(dtr, rpo[u]), rte[u]), rts[u]), corr);
             fetch(rw1[u], rw0[u], rst[u], rpo[u], rte[u], rts[u], k + D);
-            const C divided = A::rcp(A::sub(bcol, A::mul(cp, as_)));
+            const C divided = A::rcp(A::add(bcol, A::mul(cp, csp)));
             cp = A::mul(cs, divided);
-            dp = A::mul(A::sub(dv, A::mul(dp, as_)), divided);
+            dp = A::mul(A::add(dv, A::mul(dp, csp)), divided);
             fac.put(k, cp, dp);
             sprev = scur;
             scur = snext;
@@ -447,12 +447,11 @@ __device__ __forceinline__ void vadv_column(const S* __restrict__ stage, const S
     {
         const int k = nk - 1;
         o = col + (int64_t)k * sk;
-        const C as_ = A::template scale2<-1>(-gcv);
-        bcol = A::sub(dtr, as_);
+        bcol = A::add(dtr, cs);  // acol = -cs(nk-2)
         const C ddown = A::neg_diff(dup, scur, sprev);
-        corr = A::mul(-as_, ddown);
+        corr = A::mul(cs, ddown);
         dv = A::add(A::add(A::add(A::mul(dtr, ld<C, S>(pos + o)), ld<C, S>(tens + o)), ldc<C, S>(tensstage + o)), corr);
-        dp = A::div(A::sub(dv, A::mul(dp, as_)), A::sub(bcol, A::mul(cp, as_)));
+        dp = A::div(A::add(dv, A::mul(dp, cs)), A::add(bcol, A::mul(cp, cs)));
     }
 
     // ---- backward sweep
@@ -607,7 +606,7 @@ __device__ __forceinline__ void vadv_async_column(const S* __restrict__ stage, c
     C scur = ld<C, S>(stage + col + sk);
     C dup = A::sub(scur, sprev);
     C bcol = A::sub(dtr, cs);
-    C corr = A::mul(-cs, dup);
+    C corr = A::mul(A::neg(cs), dup);
     C dv = A::add(A::add(A::add(A::mul(dtr, ld<C, S>(pos + col)), ld<C, S>(tens + col)), ldc<C, S>(tensstage + col)), corr);
     P cp = AP::div(to_p<P>(cs), to_p<P>(bcol));
     P dp = AP::div(to_p<P>(dv), to_p<P>(bcol));
@@ -627,18 +626,18 @@ __device__ __forceinline__ void vadv_async_column(const S* __restrict__ stage, c
             const C snext = from_ring<C, S>(sl[2 * BT], sel_st ^ f), p0 = from_ring<C, S>(sl[3 * BT], sel_po ^ f);
             const C t0 = from_ring<C, S>(sl[4 * BT], sel_te ^ f), ts0 = from_ring<C, S>(sl[5 * BT], sel_ts ^ f);
             issue((u + D) % R, k + D);  // the slot of level k-1, already consumed
-            const C as_ = A::template scale2<-1>(-gcv);
+            const C csp = cs;  // cs(k-1) = -acol(k)
             gcv = A::template scale2<-2>(X::add(w1, w0, site<0>{}));
             cs = A::template scale2<-1>(gcv);
             const C ddown = A::neg_diff(dup, scur, sprev);
             dup = X::sub(snext, scur, site<1>{});
-            bcol = X::sub(X::sub(dtr, as_, site<2>{}), cs, site<3>{});
-            corr = X::sub(X::mul(-as_, ddown, site<4>{}), X::mul(cs, dup, site<5>{}), site<6>{});
+            bcol = X::sub(X::add(dtr, csp, site<2>{}), cs, site<3>{});
+            corr = X::sub(X::mul(csp, ddown, site<4>{}), X::mul(cs, dup, site<5>{}), site<6>{});
             dv = X::add(X::add(X::add(X::mul(dtr, p0, site<7>{}), t0, site<8>{}), ts0, site<9>{}), corr, site<10>{});
-            const P pas = to_p<P>(as_);
-            const P divided = XP::rcp(XP::sub(to_p<P>(bcol), XP::mul(cp, pas, site<11>{}), site<12>{}), site<21>{});
+            const P pcs = to_p<P>(csp);
+            const P divided = XP::rcp(XP::add(to_p<P>(bcol), XP::mul(cp, pcs, site<11>{}), site<12>{}), site<21>{});
             cp = XP::mul(to_p<P>(cs), divided, site<13>{});
-            dp = XP::mul(XP::sub(to_p<P>(dv), XP::mul(dp, pas, site<14>{}), site<15>{}), divided, site<16>{});
+            dp = XP::mul(XP::add(to_p<P>(dv), XP::mul(dp, pcs, site<14>{}), site<15>{}), divided, site<16>{});
             sc[k * FS] = cp;
             sd[k * FS] = dp;
             sprev = scur;
@@ -650,13 +649,12 @@ __device__ __forceinline__ void vadv_async_column(const S* __restrict__ stage, c
     // ---- forward sweep, k = nk-1
     {
         const IDX o = col + (IDX)(nk - 1) * sk;
-        const C as_ = A::template scale2<-1>(-gcv);
-        bcol = A::sub(dtr, as_);
+        bcol = A::add(dtr, cs);  // acol = -cs(nk-2)
         const C ddown = A::neg_diff(dup, scur, sprev);
-        corr = A::mul(-as_, ddown);
+        corr = A::mul(cs, ddown);
         dv = A::add(A::add(A::add(A::mul(dtr, ld<C, S>(pos + o)), ld<C, S>(tens + o)), ldc<C, S>(tensstage + o)), corr);
-        const P pas = to_p<P>(as_);
-        dp = AP::div(AP::sub(to_p<P>(dv), AP::mul(dp, pas)), AP::sub(to_p<P>(bcol), AP::mul(cp, pas)));
+        const P pcs = to_p<P>(cs);
+        dp = AP::div(AP::add(to_p<P>(dv), AP::mul(dp, pcs)), AP::add(to_p<P>(bcol), AP::mul(cp, pcs)));
     }
 
     // ---- backward sweep; pos of level L staged in slot (nk-2-L) % R, field 3
@@ -796,7 +794,7 @@ __device__ __forceinline__ void vadv_warp_column(const S* __restrict__ stage, co
     C scur = ld<C, S>(stage + col + sk);
     C dup = A::sub(scur, sprev);
     C bcol = A::sub(dtr, cs);
-    C corr = A::mul(-cs, dup);
+    C corr = A::mul(A::neg(cs), dup);
     C dv = A::add(A::add(A::add(A::mul(dtr, ld<C, S>(pos + col)), ld<C, S>(tens + col)), ldc<C, S>(tensstage + col)), corr);
     C cp = A::div(cs, bcol);
     C dp = A::div(dv, bcol);
@@ -816,17 +814,17 @@ __device__ __forceinline__ void vadv_warp_column(const S* __restrict__ stage, co
             const C snext = cvt<C, S>(*row(u, 2, kmis)), p0 = cvt<C, S>(*row(u, 3, kmis));
             const C t0 = cvt<C, S>(*row(u, 4, kmis)), ts0 = cvt<C, S>(*row(u, 5, kmis));
             issue((u + D) % R, k + D);  // the slot of level k-1: every lane has read it (__syncwarp above)
-            const C as_ = A::template scale2<-1>(-gcv);
+            const C csp = cs;  // cs(k-1) = -acol(k)
             gcv = A::template scale2<-2>(A::add(w1, w0));
             cs = A::template scale2<-1>(gcv);
             const C ddown = A::neg_diff(dup, scur, sprev);
             dup = A::sub(snext, scur);
-            bcol = A::sub(A::sub(dtr, as_), cs);
-            corr = A::sub(A::mul(-as_, ddown), A::mul(cs, dup));
+            bcol = A::sub(A::add(dtr, csp), cs);
+            corr = A::sub(A::mul(csp, ddown), A::mul(cs, dup));
             dv = A::add(A::add(A::add(A::mul(dtr, p0), t0), ts0), corr);
-            const C divided = A::rcp(A::sub(bcol, A::mul(cp, as_)));
+            const C divided = A::rcp(A::add(bcol, A::mul(cp, csp)));
             cp = A::mul(cs, divided);
-            dp = A::mul(A::sub(dv, A::mul(dp, as_)), divided);
+            dp = A::mul(A::add(dv, A::mul(dp, csp)), divided);
             sc[k * fs] = cp;
             sd[k * fs] = dp;
             sprev = scur;
@@ -841,12 +839,11 @@ __device__ __forceinline__ void vadv_warp_column(const S* __restrict__ stage, co
     // ---- forward sweep, k = nk-1
     {
         const IDX o = col + (IDX)(nk - 1) * sk;
-        const C as_ = A::template scale2<-1>(-gcv);
-        bcol = A::sub(dtr, as_);
+        bcol = A::add(dtr, cs);  // acol = -cs(nk-2)
         const C ddown = A::neg_diff(dup, scur, sprev);
-        corr = A::mul(-as_, ddown);
+        corr = A::mul(cs, ddown);
         dv = A::add(A::add(A::add(A::mul(dtr, ld<C, S>(pos + o)), ld<C, S>(tens + o)), ldc<C, S>(tensstage + o)), corr);
-        dp = A::div(A::sub(dv, A::mul(dp, as_)), A::sub(bcol, A::mul(cp, as_)));
+        dp = A::div(A::add(dv, A::mul(dp, cs)), A::add(bcol, A::mul(cp, cs)));
     }
 
     // ---- backward sweep: rows pos(k), ccol(k), dcol(k) of level k in slot (nk-2-k) % R
@@ -1076,7 +1073,7 @@ __device__ __forceinline__ void vadv_tmem_column(const S* __restrict__ stage, co
     C scur = ld<C, S>(stage + col + sk);
     C dup = A::sub(scur, sprev);
     C bcol = A::sub(dtr, cs);
-    C corr = A::mul(-cs, dup);
+    C corr = A::mul(A::neg(cs), dup);
     C dv = A::add(A::add(A::add(A::mul(dtr, ld<C, S>(pos + col)), ld<C, S>(tens + col)), ldc<C, S>(tensstage + col)), corr);
     C cp = A::div(cs, bcol);
     C dp = A::div(dv, bcol);
@@ -1094,17 +1091,17 @@ __device__ __forceinline__ void vadv_tmem_column(const S* __restrict__ stage, co
             const C snext = rd(u, 2, k), p0 = rd(u, 3, k);
             const C t0 = rd(u, 4, k), ts0 = rd(u, 5, k);
             issue((u + D) % R, k + D);  // the slot of level k-1: every lane has read it (__syncwarp above)
-            const C as_ = A::template scale2<-1>(-gcv);
+            const C csp = cs;  // cs(k-1) = -acol(k)
             gcv = A::template scale2<-2>(A::add(w1, w0));
             cs = A::template scale2<-1>(gcv);
             const C ddown = A::neg_diff(dup, scur, sprev);
             dup = A::sub(snext, scur);
-            bcol = A::sub(A::sub(dtr, as_), cs);
-            corr = A::sub(A::mul(-as_, ddown), A::mul(cs, dup));
+            bcol = A::sub(A::add(dtr, csp), cs);
+            corr = A::sub(A::mul(csp, ddown), A::mul(cs, dup));
             dv = A::add(A::add(A::add(A::mul(dtr, p0), t0), ts0), corr);
-            const C divided = A::rcp(A::sub(bcol, A::mul(cp, as_)));
+            const C divided = A::rcp(A::add(bcol, A::mul(cp, csp)));
             cp = A::mul(cs, divided);
-            dp = A::mul(A::sub(dv, A::mul(dp, as_)), divided);
+            dp = A::mul(A::add(dv, A::mul(dp, csp)), divided);
             tmem_st2(tcol + 2u * (uint32_t)k, cp, dp);
             sprev = scur;
             scur = snext;
@@ -1116,12 +1113,11 @@ __device__ __forceinline__ void vadv_tmem_column(const S* __restrict__ stage, co
     // ---- forward sweep, k = nk-1
     {
         const IDX o = col + (IDX)(nk - 1) * sk;
-        const C as_ = A::template scale2<-1>(-gcv);
-        bcol = A::sub(dtr, as_);
+        bcol = A::add(dtr, cs);  // acol = -cs(nk-2)
         const C ddown = A::neg_diff(dup, scur, sprev);
-        corr = A::mul(-as_, ddown);
+        corr = A::mul(cs, ddown);
         dv = A::add(A::add(A::add(A::mul(dtr, ld<C, S>(pos + o)), ld<C, S>(tens + o)), ldc<C, S>(tensstage + o)), corr);
-        dp = A::div(A::sub(dv, A::mul(dp, as_)), A::sub(bcol, A::mul(cp, as_)));
+        dp = A::div(A::add(dv, A::mul(dp, cs)), A::add(bcol, A::mul(cp, cs)));
     }
     tmem_wait_st();
 

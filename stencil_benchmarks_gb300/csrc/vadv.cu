@@ -10,7 +10,8 @@
 // Exact rewrites used to save fp64 pipe slots (all are identities in IEEE
 // arithmetic, not approximations):
 //   gav(k) = -gcv(k-1)                 both are +-0.25 * (wcon_shift[k] + wcon[k])
-//   as_ = acol, cs = ccol_raw          bet_m == bet_p == 0.5
+//   as_ = acol = -cs(k-1), cs = ccol_raw  bet_m == bet_p == 0.5; x - y * acol is
+//                                      x + y * cs(k-1), so acol is never formed
 //   x * 0.5, x * 0.25                  exponent decrements (Ar::scale2)
 //   stage[k-1] - stage[k]              negation of the previous stage[k] - stage[k-1]
 //                                      (recomputed when it is zero, to keep the sign of 0)
@@ -110,7 +111,10 @@ static_assert(kVadvDefaultIntSites == (kVadvMuls | kVadvRcpSite), "the default s
 // sequence).  Depth 1 (the next level's inputs in flight while one is
 // solved) is faster again: 742 us against 779 at depth 2, same bits.  The
 // default float64 SLAB form: depth 1, up to 28 blocks per SM, the grid
-// balanced so that every block takes the same number of groups.
+// balanced so that every block takes the same number of groups.  (Figures from
+// before the negations left the fp64 pipe, see Ar<double>::neg: the default
+// runs in 662 us since, with that pipe 63%, the ALU pipe 55% and the issue
+// slots 62% busy.)
 constexpr int kVadvPlacementDefault = 9;
 constexpr int kVadvSlabBlocksPerSm = 28;
 constexpr int kVadvPlacementCount = (int)(sizeof(kVadvPlacements) / sizeof(kVadvPlacements[0]));

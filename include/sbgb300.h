@@ -137,16 +137,19 @@ int sb_device_info(int device, char* name, int name_len, int* sm_count, int* cc_
                    int* cc_minor, size_t* total_mem, int* l2_bytes, int* smem_optin);
 int sb_synchronize(void);
 
-/* Bounded waits.  The only kernels that wait on the device are the hdiff
- * TMA tiles (SB_HDIFF_TMA), which wait on an mbarrier for each plane's tensor
- * copy.  A wait gives up after a bounded number of polls; the whole thread
- * block then stops before storing that plane, waits (bounded) for the copies
- * it still has in flight and sets a process-wide status word held in
- * page-locked, device-mapped host memory (allocated by the first TMA launch:
- * make the first sb_hdiff call before any stream capture).  The give-up is
- * reported as SB_ERR_TIMEOUT, and the word cleared, by the first of: a timed
- * sb_hdiff call (after its launch), the next sb_hdiff call (before it
- * launches anything), sb_synchronize, sb_stream_synchronize,
+/* Bounded waits.  The kernels that wait on the device are those staged by
+ * tensor copies: the hdiff TMA tiles (SB_HDIFF_TMA) and float32-compute vadv
+ * (alone and in batches), which wait on an mbarrier for each plane or block of
+ * levels.  A wait gives up after a bounded number of polls; the whole thread
+ * block (vadv: the warp) then stops before storing what it waited for, waits
+ * (bounded) for the copies it still has in flight and sets a process-wide
+ * status word held in page-locked, device-mapped host memory (allocated by the
+ * first such launch: make the first sb_hdiff call before any stream capture;
+ * sb_vadv takes a form without waits when its first call is captured).  The
+ * give-up is reported as SB_ERR_TIMEOUT, and the word cleared, by the first of:
+ * a timed sb_hdiff, sb_vadv, sb_vadv3 or sb_batch_launch call (after its
+ * launch), the next such call (before it launches anything), sb_synchronize,
+ * sb_stream_synchronize,
  * sb_event_synchronize, or sb_kernel_status.  No reference counterpart (its
  * kernels do not wait on the device).
  * sb_kernel_status: SB_ERR_TIMEOUT if a launch has given up since the last
@@ -479,6 +482,10 @@ int sb_probe_arith_rate(int kind, double* ops_per_s);
  * IEEE arithmetic.  Operands the integer path declines take the fp64
  * instruction, as in the kernels. */
 int sb_debug_soft_f64(int op, const void* a, const void* b, void* out, int64_t n, void* stream);
+/* The float32 reciprocal of the TMA-staged vadv compared on the device with the
+ * correctly rounded one for every float32 in its range: how many were checked
+ * and how many differ (synchronous). */
+int sb_debug_rcp_f32(int64_t* checked, int64_t* wrong);
 
 #ifdef __cplusplus
 }

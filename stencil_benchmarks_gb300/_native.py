@@ -158,6 +158,7 @@ SIGNATURES = {
     "sb_server_debug_launches": [_vp, _vp, _int, ctypes.POINTER(_int)],
     "sb_probe_arith_rate": [_int, _dp],
     "sb_debug_soft_f64": [_int, _vp, _vp, _vp, _i64, _vp],
+    "sb_debug_rcp_f32": [ctypes.POINTER(_i64), ctypes.POINTER(_i64)],
 }
 _RESTYPES = {"sb_last_error": ctypes.c_char_p}
 

@@ -178,16 +178,7 @@ __global__ void __launch_bounds__(512, 1)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     uint32_t* s_taddr = reinterpret_cast<uint32_t*>(smem_raw);
     unsigned char* ring = smem_raw + 16 + warp * WarpRing<S, float, D>::BYTES;
-    if (warp == 0) {
-        const uint32_t dst = (uint32_t)__cvta_generic_to_shared(s_taddr), ncols = 512u;
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(dst), "r"(ncols)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    const uint32_t tbase = *reinterpret_cast<volatile uint32_t*>(s_taddr);
+    const uint32_t tbase = tmem_alloc_all(s_taddr, warp);
     const uint32_t tcol = tbase + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)((warp >> 2) * cpw);
     for (;;) {
         unsigned long long item = 0;
@@ -218,13 +209,7 @@ __global__ void __launch_bounds__(512, 1)
                                            (const S*)dm.f[3], (const S*)dm.f[4], (S*)dm.out, col0, lane, nvalid,
                                            dm.nk, (int)dm.sk, (int)dm.wsh, tcol, ring);
     }
-    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    if (warp == 0) {
-        const uint32_t ncols = 512u;
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tbase), "r"(ncols) : "memory");
-    }
+    tmem_free_all(tbase, warp);
 }
 constexpr int kTmemDepth = 8;
 

@@ -59,6 +59,9 @@ int device_props(const DeviceProps** out);
 // returns SB_ERR_TIMEOUT (with a message) and clears the word if it was set.
 int status_word(int** device_ptr);
 int take_wait_status();
+// Whether status_word can be called for a launch on `stream`: its first call
+// allocates, which a stream under capture does not allow.
+bool status_ready(cudaStream_t stream);
 // Polls of a first wait before a thread block gives up (default 2^20; the
 // drain of copies still in flight after a give-up always uses the default).
 constexpr int kDefaultWaitPolls = 1 << 20;

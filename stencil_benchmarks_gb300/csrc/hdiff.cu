@@ -20,14 +20,11 @@
 //
 // Caller contract: inp is readable on [-2, ni+1] x [-2, nj+1] x [0, nk)
 // relative to the interior pointer (a halo of at least 2 in i and j).
-#include <cuda.h>
-#include <cudaTypedefs.h>
-
 #include <cstdlib>
-#include <mutex>
 #include <type_traits>
 
 #include "stencil_core.cuh"
+#include "tensor_map.cuh"
 
 namespace sb {
 namespace {
@@ -275,19 +272,6 @@ thread_local bool t_tma_used = false;
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t phase, int polls) {
-    for (int it = 0; it < polls; ++it) {
-        uint32_t done;
-        asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-            : "=r"(done)
-            : "r"(bar), "r"(phase)
-            : "memory");
-        if (done) return true;
-    }
-    return false;
-}
-
 __device__ __forceinline__ void tma_load_plane(const CUtensorMap* map, uint32_t dst, uint32_t bar, int x, int y,
                                                int z, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
@@ -435,28 +419,6 @@ __global__ void __launch_bounds__(TX* NTY)
             tma_load_plane(&tmap, stage0 + sidx * (uint32_t)stage, bar0 + 8 * sidx, i0, j0, k + 2, box_bytes);
         }
     }
-}
-
-PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
-    static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) ==
-                cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = (PFN_cuTensorMapEncodeTiled_v12000)p;
-        cudaGetLastError();
-    });
-    return fn;
-}
-
-template <class S>
-CUtensorMapDataType tma_type() {
-    if constexpr (sizeof(S) == 8) return CU_TENSOR_MAP_DATA_TYPE_FLOAT64;
-    else if constexpr (sizeof(S) == 4) return CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-    else return CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
 }
 
 // TMA launch if the layout qualifies (i unit-stride, j/k strides multiples

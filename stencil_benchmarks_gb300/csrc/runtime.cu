@@ -75,6 +75,16 @@ int status_word(int** device_ptr) {
     return SB_OK;
 }
 
+bool status_ready(cudaStream_t stream) {
+    if (__atomic_load_n(&g_status, __ATOMIC_ACQUIRE)) return true;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &cs) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return cs == cudaStreamCaptureStatusNone;
+}
+
 int take_wait_status() {
     if (!g_status || !__atomic_exchange_n(g_status, 0, __ATOMIC_ACQ_REL)) return SB_OK;
     return fail(SB_ERR_TIMEOUT,

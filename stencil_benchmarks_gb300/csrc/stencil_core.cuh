@@ -8,6 +8,20 @@
 
 namespace sb {
 
+// Wait for `phase` of the mbarrier at shared address `bar`, at most `polls` tries.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t phase, int polls) {
+    for (int it = 0; it < polls; ++it) {
+        uint32_t done;
+        asm volatile(
+            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+            : "=r"(done)
+            : "r"(bar), "r"(phase)
+            : "memory");
+        if (done) return true;
+    }
+    return false;
+}
+
 // ---------------------------------------------------------------------------
 // horizontal diffusion, one warp, one k-plane strip of 32 columns
 // ---------------------------------------------------------------------------
@@ -916,6 +930,29 @@ __device__ __forceinline__ void vadv_warp_column(const S* __restrict__ stage, co
 // pos rows are staged for the backward sweep.  `tcol` is the TMEM address
 // of lane 0 / column 0 of this warp's range (lane field 32 * (warp % 4)); the
 // range holds 2 * ceil(nk / 8) * 8 columns.  All 32 lanes must call this.
+// All 512 columns for the block (every warp calls it; warp 0 allocates through
+// the shared word s_taddr), and their release after the last use.
+__device__ __forceinline__ uint32_t tmem_alloc_all(uint32_t* s_taddr, int warp) {
+    if (warp == 0) {
+        const uint32_t dst = (uint32_t)__cvta_generic_to_shared(s_taddr), ncols = 512u;
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(dst), "r"(ncols)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    return *reinterpret_cast<volatile uint32_t*>(s_taddr);
+}
+__device__ __forceinline__ void tmem_free_all(uint32_t tbase, int warp) {
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    if (warp == 0) {
+        const uint32_t ncols = 512u;
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tbase), "r"(ncols) : "memory");
+    }
+}
 __device__ __forceinline__ void tmem_st2(uint32_t taddr, float a, float b) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1, %2};\n" ::"r"(taddr), "r"(__float_as_uint(a)),
                  "r"(__float_as_uint(b))

@@ -34,6 +34,8 @@
 #include <type_traits>
 
 #include "stencil_core.cuh"
+#include "tensor_map.cuh"
+#include "vadv_tma.cuh"
 
 namespace sb {
 namespace {
@@ -434,6 +436,9 @@ int launch_wslab(int bx, int depth, int blocks_per_sm, const DeviceProps* p, cud
     return SB_ERR_UNSUPPORTED;
 }
 
+// set when a launch of this thread's call contains bounded waits
+thread_local bool t_waits = false;
+
 // ---------------------------------------------------------------------------
 // TMEM variant (float32 compute): one persistent block of 4*G warps per SM.
 // Warp w solves 32-column groups with vadv_tmem_column and keeps its
@@ -466,16 +471,7 @@ __global__ void __launch_bounds__(512, 1)
     const int nwarps = blockDim.x >> 5;
     uint32_t* s_taddr = reinterpret_cast<uint32_t*>(smem_raw);
     unsigned char* ring = smem_raw + 16 + warp * WarpRing<S, float, D>::BYTES;
-    if (warp == 0) {
-        const uint32_t dst = (uint32_t)__cvta_generic_to_shared(s_taddr), ncols = 512u;
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(dst), "r"(ncols)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    const uint32_t tbase = *reinterpret_cast<volatile uint32_t*>(s_taddr);
+    const uint32_t tbase = tmem_alloc_all(s_taddr, warp);
     const uint32_t tcol = tbase + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)((warp >> 2) * cpw);
     const int gx = (ni + 31) / 32;
     const int64_t ngroups = (int64_t)gx * nj;
@@ -487,13 +483,7 @@ __global__ void __launch_bounds__(512, 1)
             vadv_tmem_column<S, D, KP, int, SA>(f.stage[c], f.pos[c], f.tens[c], f.tensstage[c], wcon, f.out[c],
                                                 i0 + j * sj, lane, nvalid, nk, sk, f.wsh[c], tcol, ring);
     }
-    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    if (warp == 0) {
-        const uint32_t ncols = 512u;
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tbase), "r"(ncols) : "memory");
-    }
+    tmem_free_all(tbase, warp);
 }
 
 // TMEM staging through 32-bit shared addresses (sb_tune.flags bit 10) or
@@ -524,6 +514,144 @@ int launch_tmem_one(int g4, int cpw, bool sa, const DeviceProps* p, cudaStream_t
     return SB_OK;
 }
 
+// ---------------------------------------------------------------------------
+// TMEM variant with TMA staging (vadv_tma.cuh): the same persistent block per
+// SM, each warp with the factors of nt level blocks in TMEM.  NC components on one wcon are
+// solved for each column group in turn, like TmemComponents.
+// ---------------------------------------------------------------------------
+template <class S, int NC>
+struct TmaArgs {
+    CUtensorMap maps[NC][kTmaFields];
+    const S* stage[NC];
+    S* out[NC];
+    int off[NC][kTmaFields];
+    int wsh[NC];
+    int ni, nj, nk, sj, sk, drift, nt, polls, stages, stage_bytes, warp_bytes;
+    int* status;
+};
+
+template <class S, int R, int NC>
+__global__ void __launch_bounds__(512, 1) vadv_tma_kernel(const __grid_constant__ TmaArgs<S, NC> a) {
+    extern __shared__ __align__(128) unsigned char smem_tma[];
+    using B = TmaBox<S, R>;
+    // warp-uniform by a broadcast, so that the tensor copies' operands can stay in uniform registers
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    const int nwarps = blockDim.x >> 5;
+    uint32_t* s_taddr = reinterpret_cast<uint32_t*>(smem_tma);
+    const uint32_t tbase = tmem_alloc_all(s_taddr, warp);
+    const uint32_t tcol = tbase + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)((warp >> 2) * a.nt * kTmaBlockCols);
+    TmaPipe<S, R> pipe;
+    unsigned char* const mem = smem_tma + B::ring_offset(nwarps) + warp * a.warp_bytes;
+    pipe.init(mem, smem_tma + 16 + warp * B::BAR_BYTES, lane, a.stages, a.stage_bytes, a.polls);
+    float* const fmem = reinterpret_cast<float*>(mem + a.stages * a.stage_bytes + kTmaPosStages * B::POSB);
+    const int gx = (a.ni + 31) / 32, ngroups = gx * a.nj;
+    const int stride = gridDim.x * nwarps;
+    auto solve_at = [&](int group, int c) {
+        TmaSolve<S> v;
+        v.live = group < ngroups;
+        const int i0 = (group % gx) * 32, j = group / gx;
+        v.maps = a.maps[c];
+#pragma unroll
+        for (int f = 0; f < kTmaFields; ++f) v.off[f] = a.off[c][f];
+        v.stage = a.stage[c];
+        v.out = a.out[c];
+        v.col0 = i0 + j * a.sj;
+        v.nvalid = min(32, a.ni - i0);
+        v.nk = a.nk;
+        v.sk = a.sk;
+        v.wsh = a.wsh[c];
+        v.drift = a.drift;
+        return v;
+    };
+    int group = blockIdx.x * nwarps + warp, c = 0;
+    TmaSolve<S> cur = solve_at(group, 0);
+    float stage0 = 0.f;
+    if (cur.live) {
+        for (int q = 0; q < a.stages; ++q) pipe.fill(cur, q);
+        stage0 = ld<float, S>(cur.stage + cur.col0 + min(lane, cur.nvalid - 1));
+    }
+    while (cur.live) {
+        if (NC == 1 || ++c == NC) {
+            c = 0;
+            group += stride;
+        }
+        const TmaSolve<S> next = solve_at(group, c);
+        if (!vadv_tma_solve<S, R>(pipe, cur, next, [&](int blk) { pipe.fill(next, blk); }, stage0, tcol,
+                                  a.nt, fmem, a.status))
+            break;
+        cur = next;
+    }
+    tmem_free_all(tbase, warp);
+}
+
+template <class S, int R, int NC>
+int launch_tma_maps(const DeviceProps* p, cudaStream_t stream, const TmemComponents<S>& comps, const void* wcon,
+                    int64_t ni, int64_t nj, int64_t nk, int64_t sj, int64_t sk) {
+    using B = TmaBox<S, R>;
+    TmaArgs<S, NC> a;
+    bool far = false;
+    for (int c = 0; c < NC; ++c) {
+        const void* const field[kTmaFields] = {wcon, comps.stage[c], comps.pos[c], comps.tens[c], comps.tensstage[c]};
+        for (const void* f : field)
+            if ((uintptr_t)f % sizeof(S)) return SB_ERR_UNSUPPORTED;
+        if (!encode_tma_maps<S, R>(a.maps[c], a.off[c], field, ni, nj, nk, sj, sk, comps.wsh[c])) return SB_ERR_UNSUPPORTED;
+        a.stage[c] = comps.stage[c];
+        a.out[c] = comps.out[c];
+        a.wsh[c] = comps.wsh[c];
+        far |= comps.wsh[c] > 1;
+    }
+    a.ni = (int)ni;
+    a.nj = (int)nj;
+    a.nk = (int)nk;
+    a.sj = (int)sj;
+    a.sk = (int)sk;
+    a.polls = wait_polls();
+    a.drift = (int)(sk * (int64_t)sizeof(S) % 16);
+    a.stage_bytes = B::stage_bytes(far);
+    const int64_t ngroups = ceil_div(ni, (int64_t)32) * nj;
+    const TmaShape shape = tma_shape<S, R>(far, nk, ngroups, p->sm_count, p->smem_optin);
+    if (shape.warps < 1) return SB_ERR_UNSUPPORTED;
+    a.stages = shape.stages;
+    a.nt = shape.nt;
+    a.warp_bytes = shape.warp_bytes;
+    // at least 120 KB: one block per SM, so the 512-column allocation is free
+    const size_t smem = std::max<size_t>(B::ring_offset(shape.warps) + (size_t)shape.warps * shape.warp_bytes, 120 * 1024);
+    const int rc = status_word(&a.status);
+    if (rc) return rc;
+    auto kernel = vadv_tma_kernel<S, R, NC>;
+    SB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int64_t grid = std::min<int64_t>(p->sm_count, ceil_div(ngroups, (int64_t)shape.warps));
+    t_waits = true;
+    kernel<<<(unsigned)grid, (unsigned)(32 * shape.warps), smem, stream>>>(a);
+    return SB_OK;
+}
+
+// TMA-staged TMEM form if this launch qualifies: float32 compute, i
+// unit-stride, positive strides, 32-bit offsets, 9 <= nk <= 256; SB_ERR_UNSUPPORTED (no error text) otherwise.
+template <class S, class C>
+int launch_tma(const DeviceProps* p, cudaStream_t stream, const TmemComponents<S>& comps, const void* wcon, int64_t ni,
+               int64_t nj, int64_t nk, int64_t si, int64_t sj, int64_t sk) {
+    if constexpr (!std::is_same<C, float>::value) {
+        return SB_ERR_UNSUPPORTED;
+    } else {
+        if (si != 1 || sj <= 0 || sk <= 0 || nk < tma_min_levels(2) || nk > 256) return SB_ERR_UNSUPPORTED;
+        const int64_t span = (ni + 1) * si + nj * sj + (nk + 1) * sk;
+        if (span >= (1LL << 31) || (int64_t)ni * nj * nk >= (1LL << 31)) return SB_ERR_UNSUPPORTED;
+        if (!status_ready(stream)) return SB_ERR_UNSUPPORTED;
+        // the map's stride: at least a granule per level, and boxes that stay inside the fields (see encode_tma_maps)
+        if (sk * (int64_t)sizeof(S) < 256) return SB_ERR_UNSUPPORTED;
+#define SB_VADV_TMA(RV)                                                                                       \
+    return comps.nc == 3 ? launch_tma_maps<S, RV, 3>(p, stream, comps, wcon, ni, nj, nk, sj, sk)               \
+                         : launch_tma_maps<S, RV, 1>(p, stream, comps, wcon, ni, nj, nk, sj, sk);
+        switch (sk * (int64_t)sizeof(S) % 16) {
+            case 0: SB_VADV_TMA(0)
+            case 8: SB_VADV_TMA(8)
+            default: SB_VADV_TMA(-1)
+        }
+#undef SB_VADV_TMA
+    }
+}
+
 // TMEM variant if this launch qualifies (float32 compute, i unit-stride,
 // positive strides, 32-bit offsets, 2 <= nk <= 256); SB_ERR_UNSUPPORTED
 // otherwise.  depth 0 = the deepest ring that fits.
@@ -550,10 +678,9 @@ int launch_tmem_comps(int depth, bool sa, const DeviceProps* p, cudaStream_t str
 }
 
 // one component
-template <class S, class C>
-int launch_tmem(int depth, bool sa, const DeviceProps* p, cudaStream_t stream, const void* stage, const void* pos,
-                const void* tens, const void* tensstage, const void* wcon, void* out, int64_t ni, int64_t nj,
-                int64_t nk, int64_t si, int64_t sj, int64_t sk, int64_t wsh) {
+template <class S>
+TmemComponents<S> one_component(const void* stage, const void* pos, const void* tens, const void* tensstage, void* out,
+                                int64_t wsh) {
     TmemComponents<S> comps{};
     comps.stage[0] = (const S*)stage;
     comps.pos[0] = (const S*)pos;
@@ -562,7 +689,14 @@ int launch_tmem(int depth, bool sa, const DeviceProps* p, cudaStream_t stream, c
     comps.out[0] = (S*)out;
     comps.wsh[0] = (int)wsh;
     comps.nc = 1;
-    return launch_tmem_comps<S, C>(depth, sa, p, stream, comps, wcon, ni, nj, nk, si, sj, sk);
+    return comps;
+}
+
+// The TMA-staged form runs for AUTO without an explicit shape and for an
+// explicit TMEM variant that names neither a ring depth nor a staging form.
+bool tma_wanted(int variant, const sb_tune* tune) {
+    if (variant == SB_VARIANT_AUTO) return !(tune && (tune->block_x || tune->block_y || tune->unroll));
+    return variant == SB_VADV_TMEM && !(tune && (tune->unroll || (tune->flags & 0xc00)));
 }
 
 template <class S, class C>
@@ -580,17 +714,21 @@ int launch_typed(const void* stage, const void* pos, const void* tens, const voi
     SB_CHECK(bx * by <= 256 && bx >= 1 && by >= 1, SB_ERR_INVALID, "vadv block (%d, %d) exceeds 256 threads", bx, by);
     const size_t smem = 2 * sizeof(C) * (size_t)nk * (size_t)(bx * by);
     const bool can_global = ccol && dcol && sizeof(S) == sizeof(C);
-    // float32 compute, no explicit shape: factors in tensor memory (512x512x80
-    // float32 137 us against 171 us for WSLAB and 180 us for SMEM async;
-    // bfloat16 113 us when the level stride is a multiple of 16 bytes, else
-    // the staging address arithmetic makes it no faster than WSLAB / SMEM).
-    // Below 2048 column groups of 32 (256 x 256) the one-block-per-SM launch
-    // is not filled and SMEM async is as fast or faster (22 vs 27 us at 64^2).
+    // float32 compute, no explicit shape: staged by TMA with factors in tensor
+    // memory at every size (figures in vadv_tma.cuh; 192 column groups of 40
+    // levels: 10.0 us on the device against 11.5 for SMEM async).  Where that
+    // form does not apply (fewer than 9 levels), row staging with factors in
+    // tensor memory from 2048 column groups of 32 on (256 x 256; below, its one
+    // block per SM is not filled), else SMEM async.
     if constexpr (std::is_same<C, float>::value) {
+        const TmemComponents<S> comps = one_component<S>(stage, pos, tens, tensstage, out, wsh);
+        if (tma_wanted(variant, tune)) {
+            const int arc = launch_tma<S, C>(p, stream, comps, wcon, ni, nj, nk, si, sj, sk);
+            if (arc != SB_ERR_UNSUPPORTED) return arc;
+        }
         if (variant == SB_VARIANT_AUTO && !(tune && (tune->block_x || tune->block_y || tune->unroll)) &&
             ceil_div(ni, (int64_t)32) * nj >= 2048 && (sizeof(S) == 4 || (sk * (int64_t)sizeof(S)) % 8 == 0)) {
-            const int arc = launch_tmem<S, C>(8, kTmemSharedAddr, p, stream, stage, pos, tens, tensstage, wcon, out,
-                                              ni, nj, nk, si, sj, sk, wsh);
+            const int arc = launch_tmem_comps<S, C>(8, kTmemSharedAddr, p, stream, comps, wcon, ni, nj, nk, si, sj, sk);
             if (arc != SB_ERR_UNSUPPORTED) return arc;
         }
     }
@@ -617,8 +755,9 @@ int launch_typed(const void* stage, const void* pos, const void* tens, const voi
         const int d = (tune && tune->unroll > 0) ? tune->unroll : 0;
         SB_CHECK(d == 0 || d == 4 || d == 8 || d == 16, SB_ERR_INVALID, "vadv TMEM ring depth must be 4, 8 or 16");
         const bool sa = tune && (tune->flags & 0x400) ? true : (tune && (tune->flags & 0x800) ? false : kTmemSharedAddr);
-        const int rc2 = launch_tmem<S, C>(d, sa, p, stream, stage, pos, tens, tensstage, wcon, out, ni, nj, nk, si, sj,
-                                          sk, wsh);
+        const int rc2 = launch_tmem_comps<S, C>(d, sa, p, stream,
+                                                one_component<S>(stage, pos, tens, tensstage, out, wsh), wcon, ni, nj,
+                                                nk, si, sj, sk);
         SB_CHECK(rc2 != SB_ERR_UNSUPPORTED, SB_ERR_UNSUPPORTED,
                  "vadv TMEM variant: needs float32 compute, i unit-stride, positive strides, 32-bit offsets and "
                  "2 <= nk <= 256");
@@ -683,7 +822,7 @@ int launch_typed3(const void* const* stage, const void* const* pos, const void* 
                                 !(tune && (tune->block_x || tune->block_y || tune->unroll)) &&
                                 ceil_div(ni, (int64_t)32) * nj >= 2048 &&
                                 (sizeof(S) == 4 || (sk * (int64_t)sizeof(S)) % 8 == 0);
-        if (auto_fused || variant == SB_VADV_TMEM) {
+        if (auto_fused || variant == SB_VADV_TMEM || tma_wanted(variant, tune)) {
             const DeviceProps* p;
             int rc = device_props(&p);
             if (rc) return rc;
@@ -697,6 +836,17 @@ int launch_typed3(const void* const* stage, const void* const* pos, const void* 
                 comps.wsh[c] = (int)wsh[c];
             }
             comps.nc = 3;
+            // the TMA form reads a component's fields while the one before it is still being written
+            bool apart = true;
+            for (int c = 0; c < 3; ++c)
+                for (int o = 0; o < 3; ++o)
+                    if (o != c && (out[c] == stage[o] || out[c] == pos[o] || out[c] == tens[o] || out[c] == tensstage[o]))
+                        apart = false;
+            if (apart && tma_wanted(variant, tune)) {
+                const int arc = launch_tma<S, C>(p, stream, comps, wcon, ni, nj, nk, si, sj, sk);
+                if (arc != SB_ERR_UNSUPPORTED) return arc;
+            }
+            if (auto_fused || variant == SB_VADV_TMEM) {
             const int d = (tune && tune->unroll > 0) ? tune->unroll : (variant == SB_VADV_TMEM ? 0 : 8);
             SB_CHECK(d == 0 || d == 4 || d == 8 || d == 16, SB_ERR_INVALID, "vadv TMEM ring depth must be 4, 8 or 16");
             const bool sa =
@@ -706,6 +856,7 @@ int launch_typed3(const void* const* stage, const void* const* pos, const void* 
             SB_CHECK(variant != SB_VADV_TMEM, SB_ERR_UNSUPPORTED,
                      "vadv TMEM variant: needs float32 compute, i unit-stride, positive strides, 32-bit offsets and "
                      "2 <= nk <= 256");
+            }
         }
     }
     for (int c = 0; c < 3; ++c) {
@@ -720,6 +871,43 @@ int launch_typed3(const void* const* stage, const void* const* pos, const void* 
 }  // namespace sb
 
 using namespace sb;
+
+// rcp_in_range against __frcp_rn over every float32 of its range
+namespace sb {
+namespace {
+__global__ void rcp_check_kernel(unsigned long long* counts) {
+    unsigned checked = 0, wrong = 0;
+    for (uint64_t b = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; b < (1ull << 32); b += (uint64_t)gridDim.x * blockDim.x) {
+        const float d = __uint_as_float((uint32_t)b);
+        if (!(fabsf(d) >= kRcpLo && fabsf(d) <= kRcpHi)) continue;
+        ++checked;
+        wrong += __float_as_uint(rcp_in_range(d)) != __float_as_uint(__frcp_rn(d));
+    }
+    atomicAdd(counts, (unsigned long long)checked);
+    atomicAdd(counts + 1, (unsigned long long)wrong);
+}
+}  // namespace
+}  // namespace sb
+
+extern "C" int sb_debug_rcp_f32(int64_t* checked, int64_t* wrong) {
+    clear_error();
+    SB_CHECK(checked && wrong, SB_ERR_INVALID, "NULL result pointer");
+    const DeviceProps* p;
+    int rc = device_props(&p);
+    if (rc) return rc;
+    unsigned long long *counts = nullptr, host[2] = {0, 0};
+    SB_CUDA(cudaMalloc(&counts, sizeof(host)));
+    cudaError_t e = cudaMemset(counts, 0, sizeof(host));
+    if (e == cudaSuccess) {
+        rcp_check_kernel<<<p->sm_count * 8, 256>>>(counts);
+        e = cudaMemcpy(host, counts, sizeof(host), cudaMemcpyDeviceToHost);
+    }
+    cudaFree(counts);
+    SB_CUDA(e);
+    *checked = (int64_t)host[0];
+    *wrong = (int64_t)host[1];
+    return SB_OK;
+}
 
 extern "C" int sb_vadv3(int storage, int compute, const void* const* stage, const void* const* pos,
                         const void* const* tens, const void* const* tensstage, const void* wcon, void* const* out,
@@ -741,8 +929,12 @@ extern "C" int sb_vadv3(int storage, int compute, const void* const* stage, cons
         return SB_OK;
     }
     SB_CHECK(nk >= 2, SB_ERR_INVALID, "vertical advection needs at least 2 levels (nk = %lld)", (long long)nk);
+    // a give-up of an earlier launch is reported before anything new runs
+    rc = take_wait_status();
+    if (rc) return rc;
     cudaStream_t s = (cudaStream_t)stream;
-    return timed(s, time_s, [&]() {
+    t_waits = false;
+    rc = timed(s, time_s, [&]() {
         if (storage == SB_F64 && compute == SB_F64)
             return launch_typed3<double, double>(stage, pos, tens, tensstage, wcon, out, ccol, dcol, ni, nj, nk, si, sj, sk, tune, s);
         if (storage == SB_F64 && compute == SB_F32X2)
@@ -753,6 +945,8 @@ extern "C" int sb_vadv3(int storage, int compute, const void* const* stage, cons
             return launch_typed3<float, double>(stage, pos, tens, tensstage, wcon, out, ccol, dcol, ni, nj, nk, si, sj, sk, tune, s);
         return launch_typed3<bf16, float>(stage, pos, tens, tensstage, wcon, out, ccol, dcol, ni, nj, nk, si, sj, sk, tune, s);
     });
+    if (rc == SB_OK && time_s && t_waits) rc = take_wait_status();
+    return rc;
 }
 
 extern "C" int sb_vadv(int storage, int compute, const void* stage, const void* pos, const void* tens,
@@ -775,8 +969,12 @@ extern "C" int sb_vadv(int storage, int compute, const void* stage, const void* 
     }
     SB_CHECK(nk >= 2, SB_ERR_INVALID, "vertical advection needs at least 2 levels (nk = %lld)", (long long)nk);
     const int64_t wsh = (int64_t)wshift_i * si + (int64_t)wshift_j * sj;
+    // a give-up of an earlier launch is reported before anything new runs
+    rc = take_wait_status();
+    if (rc) return rc;
     cudaStream_t s = (cudaStream_t)stream;
-    return timed(s, time_s, [&]() {
+    t_waits = false;
+    rc = timed(s, time_s, [&]() {
         if (storage == SB_F64 && compute == SB_F64)
             return launch_typed<double, double>(stage, pos, tens, tensstage, wcon, out, ccol, dcol, ni, nj, nk, si, sj, sk, wsh, tune, s);
         if (storage == SB_F64 && compute == SB_F32X2)
@@ -789,4 +987,6 @@ extern "C" int sb_vadv(int storage, int compute, const void* stage, const void* 
             return launch_typed<bf16, float>(stage, pos, tens, tensstage, wcon, out, ccol, dcol, ni, nj, nk, si, sj, sk, wsh, tune, s);
         return fail(SB_ERR_UNSUPPORTED, "unsupported storage/compute combination (%d, %d)", storage, compute);
     });
+    if (rc == SB_OK && time_s && t_waits) rc = take_wait_status();
+    return rc;
 }

@@ -65,7 +65,7 @@ extern "C" {
 
 /* ---- kernel variants ------------------------------------------------------ */
 #define SB_VARIANT_AUTO 0  /* the library's choice, where the layout qualifies:
-                            * hdiff: TMA for float64, VSCAN for float32, bfloat16
+                            * hdiff: SIFT for float64, VSCAN for float32, bfloat16
                             * and float pairs, JSCAN otherwise (and for fixed64);
                             * vadv: TMEM for float32 compute on >= 2048 column
                             * groups (bfloat16: level stride a multiple of 8 bytes),
@@ -80,6 +80,10 @@ extern "C" {
                            * 64 or 128 for 4-byte, 128 or 256 for 2-byte storage); i
                            * unit-stride, j/k strides multiples of the vector,
                            * inp/coeff/out at one offset from a vector boundary */
+#define SB_HDIFF_SIFT 5   /* float64 storage and compute, any layout: fluxes that the
+                           * limiter certainly zeroes are found in fixed point, the
+                           * others and the points they feed computed in float64
+                           * (no tune fields)                                       */
 #define SB_VADV_SMEM 1    /* one thread per column, ccol/dcol in shared memory     */
 #define SB_VADV_GLOBAL 2  /* one thread per column, ccol/dcol in caller scratch    */
 #define SB_VADV_SLAB 3    /* persistent threads, factors in compact per-thread slabs of

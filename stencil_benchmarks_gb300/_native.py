@@ -38,7 +38,7 @@ STREAM_GRID_STRIDE, STREAM_GRID_CHUNK = 1, 2
 BASIC_POINT, BASIC_MARCH = 1, 2
 
 VARIANT_AUTO = 0
-HDIFF_TILE, HDIFF_JSCAN, HDIFF_TMA, HDIFF_VSCAN = 1, 2, 3, 4
+HDIFF_TILE, HDIFF_JSCAN, HDIFF_TMA, HDIFF_VSCAN, HDIFF_SIFT = 1, 2, 3, 4, 5
 VADV_SMEM, VADV_GLOBAL, VADV_SLAB, VADV_WSLAB, VADV_TMEM = 1, 2, 3, 4, 5
 
 DTYPE_CODES = {"float64": SB_F64, "float32": SB_F32, "bfloat16": SB_BF16, "float32x2": SB_F32X2,

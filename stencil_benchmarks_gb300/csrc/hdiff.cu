@@ -23,6 +23,7 @@
 #include <cstdlib>
 #include <type_traits>
 
+#include "hdiff_sift.cuh"
 #include "stencil_core.cuh"
 #include "tensor_map.cuh"
 
@@ -229,6 +230,31 @@ int launch_vscan(const void* inp, const void* coeff, void* out, int64_t ni, int6
     }
 #undef SB_VSCAN_U
 #undef SB_VSCAN
+    return SB_OK;
+}
+
+// SIFT: one block per tile of 60 x 16 outputs of one plane (hdiff_sift.cuh).
+template <class IDX>
+__global__ void __launch_bounds__(32 * kSiftWarps, 9)
+    hdiff_sift_kernel(const double* __restrict__ inp, const double* __restrict__ coeff, double* __restrict__ out, int ni,
+                      int nj, IDX si, IDX sj, IDX sk) {
+    __shared__ __align__(16) SiftTile tile;
+    hdiff_sift_tile<kSiftWarps, IDX>(tile, inp, coeff, out, ni, nj, si, sj, sk, (int)blockIdx.x * kSiftOut - 2,
+                                     (int)blockIdx.y * kSiftRows, (int)blockIdx.z, threadIdx.x >> 5, threadIdx.x & 31);
+}
+
+int launch_sift(const void* inp, const void* coeff, void* out, int64_t ni, int64_t nj, int64_t nk, int64_t si, int64_t sj,
+                int64_t sk, cudaStream_t stream, const DeviceProps* p) {
+    const int64_t gx = ceil_div(ni, kSiftOut), gy = ceil_div(nj, kSiftRows);
+    if (gy > p->max_grid_y || nk > p->max_grid_z) return SB_ERR_UNSUPPORTED;
+    const dim3 grid((unsigned)gx, (unsigned)gy, (unsigned)nk), block(32 * kSiftWarps);
+    const int64_t reach = (ni + 2 + kSiftCols) * std::abs(si) + (nj + 2 + kSiftRows) * std::abs(sj) + nk * std::abs(sk);
+    if (reach < (1LL << 31))
+        hdiff_sift_kernel<int><<<grid, block, 0, stream>>>((const double*)inp, (const double*)coeff, (double*)out, (int)ni,
+                                                           (int)nj, (int)si, (int)sj, (int)sk);
+    else
+        hdiff_sift_kernel<int64_t><<<grid, block, 0, stream>>>((const double*)inp, (const double*)coeff, (double*)out,
+                                                               (int)ni, (int)nj, si, sj, sk);
     return SB_OK;
 }
 
@@ -524,10 +550,13 @@ int launch_typed(const void* inp, const void* coeff, void* out, int64_t ni, int6
     if (rc) return rc;
     int variant = tune ? tune->variant : SB_VARIANT_AUTO;
     const int placement = tune ? (tune->flags >> 4) & 15 : 0;
-    // fp64 compute is bound by the fp64 pipe: TILE computes every lap/flx/fly
-    // once per tile (fewest fp64 operations); fp32 and float-pair compute are
+    // fp64 compute is bound by the fp64 pipe.  With float64 storage SIFT leaves
+    // out what the limiter zeroes (195 us at 512x512x80, figures and worst case
+    // in hdiff_sift.cuh).  Otherwise TILE computes every lap/flx/fly once per
+    // tile (fewest fp64 operations); fp32 and float-pair compute are
     // bound by instruction issue: JSCAN (shuffles, no block barriers) is faster.
-    // With float64 storage too, the TMA-staged tile is faster still (its
+    // With a placement preset of its sites asked for, or a domain too large for
+    // SIFT's grid, the TMA-staged tile is the fastest that computes everything (its
     // loads leave the issue slots to the fp64 arithmetic and overlap the
     // previous plane's compute); it needs TMA-describable strides, else TILE.
     // 128 x 4 threads, 16-row tiles, one k-plane per block at 512x512x80:
@@ -535,6 +564,12 @@ int launch_typed(const void* inp, const void* coeff, void* out, int64_t ni, int6
     // 24 and 32 rows 652-716 (two blocks per SM no longer fit).
     const bool auto_tile = variant == SB_VARIANT_AUTO && std::is_same<C, double>::value;
     if constexpr (std::is_same<S, double>::value && std::is_same<C, double>::value) {
+        if (variant == SB_HDIFF_SIFT || (variant == SB_VARIANT_AUTO && placement == 0)) {
+            const int rc_sift = launch_sift(inp, coeff, out, ni, nj, nk, si, sj, sk, stream, p);
+            SB_CHECK(rc_sift != SB_ERR_UNSUPPORTED || variant == SB_VARIANT_AUTO, SB_ERR_UNSUPPORTED,
+                     "hdiff SIFT: domain too large for its launch grid");
+            if (rc_sift != SB_ERR_UNSUPPORTED) return rc_sift;
+        }
         if (variant == SB_VARIANT_AUTO) {
             const int rc_tma =
                 launch_tma_placed<S, C, 128, 4>(placement, inp, coeff, out, ni, nj, nk, si, sj, sk, 16, 1, stream, p);
@@ -561,6 +596,7 @@ int launch_typed(const void* inp, const void* coeff, void* out, int64_t ni, int6
     if constexpr (std::is_same<C, fix64>::value) {
         SB_CHECK(variant == SB_HDIFF_JSCAN, SB_ERR_UNSUPPORTED, "fixed-point hdiff runs as JSCAN strips only");
     }
+    SB_CHECK(variant != SB_HDIFF_SIFT, SB_ERR_UNSUPPORTED, "hdiff SIFT needs float64 storage and compute");
     SB_CHECK(variant == SB_HDIFF_TILE || variant == SB_HDIFF_JSCAN || variant == SB_HDIFF_TMA ||
                  variant == SB_HDIFF_VSCAN,
              SB_ERR_UNSUPPORTED, "hdiff variant %d is not available", variant);

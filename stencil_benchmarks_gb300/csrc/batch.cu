@@ -12,9 +12,10 @@
 //
 // hdiff: persistent warps; an item is a strip of 28 output columns x `rows`
 //   rows x `planes` k-planes of one domain (stencil_core.cuh:
+//   hdiff_vscan_strip where the rows take aligned vectors, else
 //   hdiff_jscan_strip).  A warp takes the next item with one atomicAdd and
-//   finds its domain by binary search over first-item offsets staged in
-//   shared memory.
+//   finds its domain by binary search over the first-item offsets.  Exact
+//   float64: blocks take 60 x 16 tiles x `planes` planes (hdiff_sift.cuh).
 // vadv: persistent blocks of BT threads; an item is BT consecutive columns of
 //   one j-row of one domain, one column per thread (stencil_core.cuh:
 //   vadv_async_column: cp.async-staged inputs).  Factors live in shared memory
@@ -23,13 +24,18 @@
 //   frees shared memory for more blocks per SM.  Domains are grouped into 8 nk
 //   buckets (caps max_nk/8, 2*max_nk/8, ...) and each bucket's kernel and slab
 //   are sized for its cap, so short columns do not pay for the tallest one.
+//   With float32 arithmetic, i unit-stride and no column shorter than 17 levels
+//   all vadv domains run in one kernel instead, staged by TMA from one queue
+//   (batch_vadv_tma_kernel).
 // No kernel waits on another warp or kernel: every queue is one atomic counter.
 #include <algorithm>
 #include <cstring>
 #include <type_traits>
 #include <vector>
 
+#include "hdiff_sift.cuh"
 #include "stencil_core.cuh"
+#include "vadv_tma.cuh"
 
 namespace sb {
 namespace {
@@ -46,9 +52,13 @@ struct DevDomain {
     void* out;
     int64_t item_begin;  // first item of this domain in its queue
     int32_t items_i, items_j;
-    int32_t kp;  // vadv: level stride 0 (1) or 8 (2) modulo 16 bytes, else 0 (TMEM staging shortcuts)
-    int32_t pad;
+    int32_t kp;   // vadv: level stride 0 (1) or 8 (2) modulo 16 bytes, else 0 (TMEM staging shortcuts)
+    int32_t vec;  // hdiff: aligned vectors of the strip form fit this domain's rows
+    int32_t cs0;  // ... first column of strip 0 then
+    int32_t drift, off[kTmaFields];  // vadv by TMA (vadv_tma.cuh)
+    CUtensorMap maps[kTmaFields];
 };
+static_assert(alignof(DevDomain) % 64 == 0, "tensor maps lie on 64-byte boundaries");
 
 struct DevTable {
     int32_t ndomains, n_hdiff;
@@ -62,41 +72,93 @@ struct DevTable {
 
 size_t table_bytes(int n) { return offsetof(DevTable, dom) + sizeof(DevDomain) * (size_t)(n > 0 ? n : 1); }
 
+// columns per lane of the vector strips (as the single-domain kernel), 0 where strips of one column stay
+template <class S, class C>
+constexpr int kBatchV = std::is_same<C, fix64>::value || (sizeof(S) != sizeof(C) && sizeof(S) == 4) ? 0
+                        : sizeof(S) == 2                                                           ? 4
+                                                                                                   : 2;
+// output columns of a strip
+template <class S, class C>
+constexpr int kBatchStep = kBatchV<S, C> == 0 ? kJscanOut
+                                              : 32 * kBatchV<S, C> - kBatchV<S, C> * ((4 + kBatchV<S, C> - 1) / (kBatchV<S, C> == 0 ? 1 : kBatchV<S, C>));
+
+// the domain of an item among [lo, hi]: the last one whose first item is not past it
+__device__ __forceinline__ int find_domain(const DevTable* __restrict__ tab, int lo, int hi, int64_t item) {
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (tab->dom[mid].item_begin <= item) lo = mid; else hi = mid - 1;
+    }
+    return lo;
+}
+
 template <class S, class C, int U, class IDX>
 __global__ void __launch_bounds__(256)
     batch_hdiff_kernel(const DevTable* __restrict__ tab, unsigned long long* __restrict__ counter) {
-    __shared__ int64_t s_begin[kMaxBatchDomains + 1];
     const int nd = tab->n_hdiff;
     const int64_t total = tab->hdiff_items;
     if (total == 0) return;
     const int rows = tab->rows, planes = tab->planes;
-    for (int d = threadIdx.x; d < nd; d += blockDim.x) s_begin[d] = tab->dom[d].item_begin;
-    if (threadIdx.x == 0) s_begin[nd] = total;
-    __syncthreads();
     const int lane = threadIdx.x & 31;
     for (;;) {
         unsigned long long item = 0;
         if (lane == 0) item = atomicAdd(counter, 1ULL);
         item = __shfl_sync(0xffffffffu, item, 0);
         if ((int64_t)item >= total) break;
-        int lo = 0, hi = nd - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (s_begin[mid] <= (int64_t)item) lo = mid; else hi = mid - 1;
-        }
-        const DevDomain& dm = tab->dom[lo];
-        const int64_t local = (int64_t)item - s_begin[lo];
+        const int d = find_domain(tab, 0, nd - 1, (int64_t)item);
+        const DevDomain& dm = tab->dom[d];
+        const int64_t local = (int64_t)item - dm.item_begin;
         const int strip = (int)(local % dm.items_i);
         const int64_t rest = local / dm.items_i;
         const int jb = (int)(rest % dm.items_j);
         const int k0 = (int)(rest / dm.items_j) * planes;
         const int k1 = min(dm.nk, k0 + planes);
-        const int i = strip * kJscanOut - 2 + lane;
         const int j0 = jb * rows;
         const int j1 = min(dm.nj, j0 + rows);
+        if constexpr (kBatchV<S, C> > 0) {
+            if (dm.vec) {
+                constexpr int V = kBatchV<S, C>, step = kBatchStep<S, C>;
+                for (int k = k0; k < k1; ++k)
+                    hdiff_vscan_strip<S, C, V, (V == 4 ? 1 : U), IDX>((const S*)dm.f[0], (const S*)dm.f[1], (S*)dm.out,
+                                                                      dm.ni, dm.nj, (IDX)dm.sj, (IDX)dm.sk,
+                                                                      dm.cs0 + strip * step, step, lane, j0, j1, k);
+                continue;
+            }
+        }
+        const int i = strip * kJscanOut - 2 + lane;
         for (int k = k0; k < k1; ++k) {
             hdiff_strip<S, C, U, IDX>((const S*)dm.f[0], (const S*)dm.f[1], (S*)dm.out, dm.ni, dm.nj,
                                             (IDX)dm.si, (IDX)dm.sj, (IDX)dm.sk, i, lane, j0, j1, k);
+        }
+    }
+}
+
+// Exact float64: blocks take 60 x 16 tiles (hdiff_sift.cuh).
+template <class IDX>
+__global__ void __launch_bounds__(32 * kSiftWarps, 9)
+    batch_sift_kernel(const DevTable* __restrict__ tab, unsigned long long* __restrict__ counter) {
+    __shared__ __align__(16) SiftTile tile;
+    __shared__ int64_t s_item;
+    const int64_t total = tab->hdiff_items;
+    if (total == 0) return;
+    const int nd = tab->n_hdiff, planes = tab->planes;
+    for (;;) {
+        __syncthreads();  // the tile and s_item are free again
+        if (threadIdx.x == 0) s_item = (int64_t)atomicAdd(counter, 1ULL);
+        __syncthreads();
+        const int64_t item = s_item;
+        if (item >= total) break;
+        const DevDomain& dm = tab->dom[find_domain(tab, 0, nd - 1, item)];
+        const int64_t local = item - dm.item_begin;
+        const int strip = (int)(local % dm.items_i);
+        const int64_t rest = local / dm.items_i;
+        const int jb = (int)(rest % dm.items_j);
+        const int k0 = (int)(rest / dm.items_j) * planes;
+        const int k1 = min(dm.nk, k0 + planes);
+        for (int k = k0; k < k1; ++k) {
+            if (k > k0) __syncthreads();
+            hdiff_sift_tile<kSiftWarps, IDX>(tile, (const double*)dm.f[0], (const double*)dm.f[1], (double*)dm.out, dm.ni,
+                                             dm.nj, (IDX)dm.si, (IDX)dm.sj, (IDX)dm.sk, strip * kSiftOut - 2,
+                                             jb * kSiftRows, k, threadIdx.x >> 5, threadIdx.x & 31);
         }
     }
 }
@@ -125,13 +187,8 @@ __global__ void __launch_bounds__(BT)
             const int64_t item = (int64_t)atomicAdd(counter, 1ULL);
             int d = -1;
             if (item < total) {
-                int lo = first, hi = last - 1;
-                while (lo < hi) {
-                    const int mid = (lo + hi + 1) >> 1;
-                    if (tab->dom[mid].item_begin <= item) lo = mid; else hi = mid - 1;
-                }
-                d = lo;
-                s_local = item - tab->dom[lo].item_begin;
+                d = find_domain(tab, first, last - 1, item);
+                s_local = item - tab->dom[d].item_begin;
             }
             s_dom = d;
         }
@@ -185,12 +242,7 @@ __global__ void __launch_bounds__(512, 1)
         if (lane == 0) item = atomicAdd(counter, 1ULL);
         item = __shfl_sync(0xffffffffu, item, 0);
         if ((int64_t)item >= total) break;  // whole warp
-        int lo = first, hi = last - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (tab->dom[mid].item_begin <= (int64_t)item) lo = mid; else hi = mid - 1;
-        }
-        const DevDomain& dm = tab->dom[lo];
+        const DevDomain& dm = tab->dom[find_domain(tab, first, last - 1, (int64_t)item)];
         const int64_t local = (int64_t)item - dm.item_begin;
         const int i0 = (int)(local % dm.items_i) * 32;
         const int j = (int)(local / dm.items_i);
@@ -213,6 +265,87 @@ __global__ void __launch_bounds__(512, 1)
 }
 constexpr int kTmemDepth = 8;
 
+// float32-compute vadv staged by TMA (vadv_tma.cuh): one persistent block per SM
+// for all vadv domains of the set, whatever their nk; its warps take 32-column
+// items from one queue, tallest domains first.  One kernel instead of one per
+// bucket: each of those fills every SM's TMEM, so they ran one after the other,
+// each with its own last round.
+struct TmaBatch {
+    int nt, stages, stage_bytes, warp_bytes, polls;
+    int* status;
+};
+template <class S, int R>
+__global__ void __launch_bounds__(512, 1)
+    batch_vadv_tma_kernel(const DevTable* __restrict__ tab, unsigned long long* __restrict__ counter, const TmaBatch a) {
+    extern __shared__ __align__(128) unsigned char smem_tma[];
+    using B = TmaBox<S, R>;
+    const int first = tab->bucket_first[0], last = tab->bucket_first[kBuckets];
+    const int64_t total = tab->bucket_items[0];
+    if (total == 0) return;  // whole block, before any TMEM allocation
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    const int nwarps = blockDim.x >> 5;
+    const uint32_t tbase = tmem_alloc_all(reinterpret_cast<uint32_t*>(smem_tma), warp);
+    const uint32_t tcol = tbase + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)((warp >> 2) * a.nt * kTmaBlockCols);
+    TmaPipe<S, R> pipe;
+    unsigned char* const mem = smem_tma + B::ring_offset(nwarps) + warp * a.warp_bytes;
+    pipe.init(mem, smem_tma + 16 + warp * B::BAR_BYTES, lane, a.stages, a.stage_bytes, a.polls);
+    float* const fmem = reinterpret_cast<float*>(mem + a.stages * a.stage_bytes + kTmaPosStages * B::POSB);
+    int known = -1;  // domain whose maps this warp has acquired last
+    auto take = [&]() {
+        TmaSolve<S> v;
+        unsigned long long item = 0;
+        if (lane == 0) item = atomicAdd(counter, 1ULL);
+        item = __shfl_sync(0xffffffffu, item, 0);
+        v.live = (int64_t)item < total;
+        const int lo = v.live ? find_domain(tab, first, last - 1, (int64_t)item) : first;
+        const DevDomain& dm = tab->dom[lo];
+        const int local = (int)((int64_t)item - dm.item_begin);
+        const int i0 = v.live ? (local % dm.items_i) * 32 : 0, j = v.live ? local / dm.items_i : 0;
+        v.maps = dm.maps;
+#pragma unroll
+        for (int f = 0; f < kTmaFields; ++f) v.off[f] = dm.off[f];
+        v.stage = (const S*)dm.f[0];
+        v.out = (S*)dm.out;
+        v.col0 = i0 + j * (int)dm.sj;
+        v.nvalid = min(32, dm.ni - i0);
+        v.nk = dm.nk;
+        v.sk = (int)dm.sk;
+        v.wsh = (int)dm.wsh;
+        v.drift = dm.drift;
+        if (v.live && lo != known) {
+            acquire_maps(v.maps);
+            known = lo;
+        }
+        return v;
+    };
+    TmaSolve<S> cur = take();
+    float stage0 = 0.f;
+    if (cur.live) {
+        for (int q = 0; q < a.stages; ++q) pipe.fill(cur, q);
+        stage0 = ld<float, S>(cur.stage + cur.col0 + min(lane, cur.nvalid - 1));
+    }
+    while (cur.live) {
+        const TmaSolve<S> next = take();
+        if (!vadv_tma_solve<S, R>(pipe, cur, next, [&](int blk) { pipe.fill(next, blk); }, stage0, tcol, a.nt, fmem,
+                                  a.status))
+            break;
+        cur = next;
+    }
+    tmem_free_all(tbase, warp);
+}
+
+// the TMA form for level strides of one drift class: 0, 8 or any bytes modulo 16
+constexpr int kTmaClasses = 3;
+struct TmaClass {
+    void (*run)(dim3, dim3, size_t, cudaStream_t, const DevTable*, unsigned long long*, const TmaBatch&);
+    const void* fn;
+    TmaShape (*shape)(bool far, int64_t max_nk, int sms, int smem_optin);
+    bool (*encode)(CUtensorMap*, int*, const void* const (&)[kTmaFields], int64_t, int64_t, int64_t, int64_t, int64_t,
+                   int64_t);
+    int (*stage_bytes)(bool far);
+    int (*ring_offset)(int nwarps);
+};
+
 struct Kinds {
     void (*hdiff)(dim3, dim3, cudaStream_t, const DevTable*, unsigned long long*);
     void (*vadv32)(dim3, dim3, size_t, cudaStream_t, const DevTable*, unsigned long long*, int, int, int, void*);
@@ -227,6 +360,9 @@ struct Kinds {
     void (*vadv_tmem)(dim3, dim3, size_t, cudaStream_t, const DevTable*, unsigned long long*, int, int);
     const void* vadv_tmem_fn;
     int tmem_ring_bytes;  // staging ring per warp
+    TmaClass tma[kTmaClasses];  // run == nullptr for other compute types
+    bool sift;                  // hdiff blocks take SIFT tiles
+    int hdiff_v, hdiff_step;    // vector strips: columns per lane (0: none) and output columns
 };
 
 template <class S, class C, int U, class IDX>
@@ -251,6 +387,26 @@ void run_vadv_tmem(dim3 g, dim3 b, size_t smem, cudaStream_t s, const DevTable* 
     batch_vadv_tmem_kernel<S, kTmemDepth><<<g, b, smem, s>>>(t, c, bucket, cpw);
 }
 
+template <class S, int R>
+TmaClass tma_class() {
+    TmaClass c;
+    c.run = [](dim3 g, dim3 b, size_t smem, cudaStream_t s, const DevTable* t, unsigned long long* q, const TmaBatch& a) {
+        batch_vadv_tma_kernel<S, R><<<g, b, smem, s>>>(t, q, a);
+    };
+    c.fn = (const void*)&batch_vadv_tma_kernel<S, R>;
+    // the most warps (a batch has more column groups than any launch has warps)
+    c.shape = [](bool far, int64_t max_nk, int sms, int optin) {
+        return tma_shape<S, R>(far, max_nk, (int64_t)1 << 40, sms, optin);
+    };
+    c.encode = [](CUtensorMap* m, int* off, const void* const (&f)[kTmaFields], int64_t ni, int64_t nj, int64_t nk,
+                  int64_t sj, int64_t sk, int64_t wsh) {
+        return encode_tma_maps<S, R>(m, off, f, ni, nj, nk, sj, sk, wsh);
+    };
+    c.stage_bytes = [](bool far) { return TmaBox<S, R>::stage_bytes(far); };
+    c.ring_offset = [](int n) { return TmaBox<S, R>::ring_offset(n); };
+    return c;
+}
+
 // hdiff computes in HC, vadv in VC with its recurrences in P
 template <class S, class HC, class VC, int U, class IDX, class P = VC>
 Kinds kinds_for() {
@@ -260,7 +416,15 @@ Kinds kinds_for() {
     constexpr bool SLAB = sizeof(typename RingOf<S>::T) == sizeof(P) &&
                           !(std::is_same<S, float>::value && std::is_same<P, float>::value);
     k.slab = SLAB;
-    k.hdiff = &run_hdiff<S, HC, U, IDX>;
+    k.sift = std::is_same<S, double>::value && std::is_same<HC, double>::value;
+    k.hdiff_v = k.sift ? 0 : kBatchV<S, HC>;
+    k.hdiff_step = kBatchStep<S, HC>;
+    if constexpr (std::is_same<S, double>::value && std::is_same<HC, double>::value)
+        k.hdiff = [](dim3 g, dim3, cudaStream_t s, const DevTable* t, unsigned long long* c) {
+            batch_sift_kernel<IDX><<<g, 32 * kSiftWarps, 0, s>>>(t, c);
+        };
+    else
+        k.hdiff = &run_hdiff<S, HC, U, IDX>;
     // float64 slab buckets: the single-domain kernel's split between the fp64
     // and integer pipes (more blocks per SM, below)
     constexpr uint32_t PL = SLAB && std::is_same<P, double>::value && std::is_same<VC, double>::value
@@ -278,10 +442,14 @@ Kinds kinds_for() {
         k.vadv_tmem = &run_vadv_tmem<S>;
         k.vadv_tmem_fn = (const void*)&batch_vadv_tmem_kernel<S, kTmemDepth>;
         k.tmem_ring_bytes = WarpRing<S, float, kTmemDepth>::BYTES;
+        k.tma[0] = tma_class<S, 0>();
+        k.tma[1] = tma_class<S, 8>();
+        k.tma[2] = tma_class<S, -1>();
     } else {
         k.vadv_tmem = nullptr;
         k.vadv_tmem_fn = nullptr;
         k.tmem_ring_bytes = 0;
+        for (auto& c : k.tma) c = TmaClass{};
     }
     return k;
 }
@@ -339,6 +507,12 @@ struct sb_batch {
     int tmem_block[kBuckets] = {}, tmem_cpw[kBuckets] = {};
     int vadv_tmem_grid = 0;
     size_t tmem_smem = 0;
+    // float32 vadv staged by TMA: what the current domain set uses and what the captured graph has
+    // (drift class + kTmaClasses where a domain reads wcon at j + 1; -1: not this form)
+    int use_tma = -1, graph_tma = -1;
+    TmaShape tma_shapes[2 * kTmaClasses] = {};
+    int* status = nullptr;
+    int graph_polls = 0;
 };
 
 namespace {
@@ -365,6 +539,39 @@ size_t vadv_smem_bytes(int cap, int bt, int cbytes, int sbytes, int depth, int* 
     return fac + (size_t)(depth + 1) * 6 * bt * sbytes;
 }
 
+// Drift class of the set's vadv domains (see sb_batch::use_tma) where the TMA
+// form takes all of them, else -1.
+int tma_of_set(const sb_batch* b, const Kinds& k, const sb_domain* domains, const std::vector<int> (&vd)[kBuckets]) {
+    if (!k.tma[0].run) return -1;
+    const int es = storage_size(b->storage);
+    int cls = 0;
+    bool far = false;
+    int64_t min_nk = 1 << 30;
+    for (const auto& v : vd) {
+        for (int q : v) {
+            const sb_domain& s = domains[q];
+            if (s.ni == 0 || s.nj == 0) continue;
+            if (s.si != 1 || s.sj <= 0 || s.sk <= 0 || s.sk * es < 256) return -1;
+            if ((s.ni + 33) + (s.nj + 2) * s.sj + (s.nk + 1) * s.sk >= (1LL << 31)) return -1;
+            for (const void* f : s.f)
+                if ((uintptr_t)f % es) return -1;
+            const int64_t drift = s.sk * es % 16;
+            if (drift != 0) cls = std::max(cls, drift == 8 ? 1 : 2);
+            far |= (int64_t)s.wshift_j * s.sj > 1;
+            min_nk = std::min(min_nk, s.nk);
+        }
+    }
+    // one exact class for the whole set: drift 0 and 8 together are "any"
+    if (cls == 1)
+        for (const auto& v : vd)
+            for (int q : v)
+                if (domains[q].ni && domains[q].nj && domains[q].sk * es % 16 == 0) cls = 2;
+    const int use = cls + (far ? kTmaClasses : 0);
+    const TmaShape& sh = b->tma_shapes[use];
+    if (sh.warps < 1 || min_nk < tma_min_levels(sh.stages)) return -1;
+    return use;
+}
+
 int capture_graph(sb_batch* b) {
     if (b->exec) {
         cudaGraphExecDestroy(b->exec);
@@ -382,7 +589,16 @@ int capture_graph(sb_batch* b) {
         if (b->vadv_smem[q] > 48 * 1024)
             SB_CUDA(cudaFuncSetAttribute(vadv_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->vadv_smem[q]));
     }
-    if (b->use_tmem)
+    TmaBatch ta{};
+    size_t tma_smem = 0;
+    if (b->use_tma >= 0) {
+        const TmaClass& c = k.tma[b->use_tma % kTmaClasses];
+        const TmaShape& sh = b->tma_shapes[b->use_tma];
+        ta = {sh.nt, sh.stages, c.stage_bytes(b->use_tma >= kTmaClasses), sh.warp_bytes, wait_polls(), b->status};
+        tma_smem = std::max<size_t>(c.ring_offset(sh.warps) + (size_t)sh.warps * sh.warp_bytes, 120 * 1024);
+        SB_CUDA(cudaFuncSetAttribute(c.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tma_smem));
+        b->graph_polls = ta.polls;
+    } else if (b->use_tmem)
         SB_CUDA(cudaFuncSetAttribute(k.vadv_tmem_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->tmem_smem));
     cudaStream_t s0 = b->streams[0];
     SB_CUDA(cudaStreamBeginCapture(s0, cudaStreamCaptureModeThreadLocal));
@@ -391,15 +607,26 @@ int capture_graph(sb_batch* b) {
     cudaEventRecord(b->fork, s0);
     // order 0: hdiff first, then the vadv buckets; order 1: the vadv buckets
     // first (tallest first), so their blocks are resident before the hdiff
-    // blocks take the remaining room of each SM
-    const bool vadv_first = b->tune.order == 1;
+    // blocks take the remaining room of each SM.  The TMA form, whose one block
+    // per SM otherwise waits for that room, always goes first (64 uneven
+    // domains: float32 1321 us against 1454, bfloat16 1158 against 1532; the
+    // float64 slab buckets gain nothing from it, 980 against 832 for 8 domains).
+    const bool vadv_first = b->tune.order == 1 || b->use_tma >= 0;
     auto launch_hdiff = [&]() {
         cudaStreamWaitEvent(b->streams[1], b->fork, 0);
         k.hdiff(dim3(b->hdiff_grid), dim3(b->hdiff_block), b->streams[1], b->dev_table, b->counters);
         cudaEventRecord(b->joins[0], b->streams[1]);
     };
     if (!vadv_first) launch_hdiff();
-    for (int qq = 0; qq < kBuckets; ++qq) {
+    const int nvadv = b->use_tma >= 0 ? 1 : kBuckets;  // vadv kernels
+    for (int qq = 0; qq < nvadv; ++qq) {
+        if (nvadv == 1) {
+            cudaStreamWaitEvent(b->streams[2], b->fork, 0);
+            k.tma[b->use_tma % kTmaClasses].run(dim3(b->vadv_tmem_grid), dim3(32 * b->tma_shapes[b->use_tma].warps),
+                                                tma_smem, b->streams[2], b->dev_table, b->counters + 1, ta);
+            cudaEventRecord(b->joins[1], b->streams[2]);
+            break;
+        }
         const int q = vadv_first ? kBuckets - 1 - qq : qq;
         cudaStreamWaitEvent(b->streams[2 + q], b->fork, 0);
         if (b->use_tmem)
@@ -411,7 +638,7 @@ int capture_graph(sb_batch* b) {
         cudaEventRecord(b->joins[1 + q], b->streams[2 + q]);
     }
     if (vadv_first) launch_hdiff();
-    for (int q = 0; q < 1 + kBuckets; ++q) cudaStreamWaitEvent(s0, b->joins[q], 0);
+    for (int q = 0; q < 1 + nvadv; ++q) cudaStreamWaitEvent(s0, b->joins[q], 0);
     cudaGraph_t graph = nullptr;
     const cudaError_t ec = cudaStreamEndCapture(s0, &graph);
     if (ec != cudaSuccess) {
@@ -422,6 +649,7 @@ int capture_graph(sb_batch* b) {
     SB_CUDA(cudaGraphInstantiate(&b->exec, graph, 0));
     b->graph_idx64 = b->idx64;
     b->graph_tmem = b->use_tmem;
+    b->graph_tma = b->use_tma;
     return SB_OK;
 }
 
@@ -451,7 +679,9 @@ int sb_batch_create(sb_batch** out, int storage, int compute, int max_domains, i
     b->max_nk = max_nk;
     if (tune) b->tune = *tune;
     b->hdiff_block = b->tune.block > 0 ? b->tune.block : 128;
-    const int per_sm = b->tune.blocks_per_sm > 0 ? b->tune.blocks_per_sm : 4;
+    // 8 blocks per SM: 64 uneven domains, half of them hdiff, float32 1419 us (the
+    // hdiff ones alone 544) against 1678 (774) with 4; bfloat16 1443 against 2062
+    const int per_sm = b->tune.blocks_per_sm > 0 ? b->tune.blocks_per_sm : 8;
     b->vadv_block = b->tune.vadv_block > 0 ? b->tune.vadv_block : 32;
     if (b->hdiff_block % 32 || b->hdiff_block > 256 || per_sm > 32 || (b->vadv_block != 32 && b->vadv_block != 64)) {
         release(b);
@@ -461,6 +691,7 @@ int sb_batch_create(sb_batch** out, int storage, int compute, int max_domains, i
     if (b->tune.hdiff_rows <= 0) b->tune.hdiff_rows = 32;
     if (b->tune.hdiff_planes <= 0) b->tune.hdiff_planes = 1;
     b->hdiff_grid = p->sm_count * per_sm;
+    if (k.sift && b->tune.blocks_per_sm <= 0) b->hdiff_grid = p->sm_count * 12;
     for (int q = 0; q < kBuckets; ++q) {
         b->cap[q] = (int)std::max<int64_t>(2, ceil_div(max_nk * (q + 1), kBuckets));
         // slab mode: shared memory holds the ring only (cap 0 factor levels)
@@ -500,6 +731,14 @@ int sb_batch_create(sb_batch** out, int storage, int compute, int max_domains, i
         }
         b->tmem_smem = smem;
         b->vadv_tmem_grid = p->sm_count;
+        for (int q = 0; q < 2 * kTmaClasses; ++q)
+            if (k.tma[q % kTmaClasses].run && max_nk >= tma_min_levels(2))
+                b->tma_shapes[q] = k.tma[q % kTmaClasses].shape(q >= kTmaClasses, max_nk, p->sm_count, p->smem_optin);
+        rc = status_word(&b->status);
+        if (rc) {
+            release(b);
+            return rc;
+        }
     }
     size_t slab_total = 0;
     size_t slab_off[kBuckets] = {};
@@ -581,9 +820,13 @@ int sb_batch_set(sb_batch* b, const sb_domain* domains, int n) {
         std::stable_sort(v.begin(), v.end(), [&](int x, int y) { return domains[x].nk > domains[y].nk; });
     bool idx64 = false;
     bool tmem_ok = b->tmem_capable;
+    Kinds k;
+    SB_CHECK(pick_kinds(b->storage, b->compute, false, &k), SB_ERR_UNSUPPORTED, "unsupported form");
+    int tma = b->tmem_capable ? tma_of_set(b, k, domains, vd) : -1;
     const int es = storage_size(b->storage);
     DevTable* t = b->host_table;
     int slot = 0;
+    bool encoded = true;
     auto fill = [&](int q, int64_t& items) {
         const sb_domain& s = domains[q];
         DevDomain& d = t->dom[slot++];
@@ -603,34 +846,77 @@ int sb_batch_set(sb_batch* b, const sb_domain* domains, int n) {
         if (s.ni == 0 || s.nj == 0 || s.nk == 0) return;
         if (s.op == SB_OP_HDIFF) {
             d.items_i = (int32_t)ceil_div(s.ni, kJscanOut);
-            d.items_j = (int32_t)ceil_div(s.nj, b->tune.hdiff_rows);
+            d.items_j = (int32_t)ceil_div(s.nj, k.sift ? kSiftRows : b->tune.hdiff_rows);
+            if (k.sift) {
+                d.items_i = (int32_t)ceil_div(s.ni, kSiftOut);
+            } else if (k.hdiff_v) {
+                // aligned vectors of V columns: as launch_vscan of the single-domain kernel
+                const int V = k.hdiff_v, VB = V * es;
+                const uintptr_t at = (uintptr_t)s.f[0];
+                d.vec = s.si == 1 && s.sj > 0 && s.sk > 0 && (s.sj * es) % VB == 0 && (s.sk * es) % VB == 0 && at % es == 0 &&
+                        (uintptr_t)s.f[1] % VB == at % VB && (uintptr_t)s.out % VB == at % VB;
+                if (d.vec) {
+                    const int off = (int)((at % VB) / es);
+                    d.cs0 = -2 - (((off - 2) % V) + V) % V;
+                    d.items_i = (int32_t)ceil_div(s.ni - (d.cs0 + 2), (int64_t)k.hdiff_step);
+                }
+            }
             items += (int64_t)d.items_i * d.items_j * ceil_div(s.nk, b->tune.hdiff_planes);
         } else {
             d.wsh = (int64_t)s.wshift_i * s.si + (int64_t)s.wshift_j * s.sj;
             d.kp = (s.sk * es) % 16 == 0 ? 1 : (s.sk * es) % 16 == 8 ? 2 : 0;
             if (s.si != 1 || s.sj <= 0 || s.sk <= 0) tmem_ok = false;
+            if (tma >= 0) {
+                const void* const field[kTmaFields] = {s.f[4], s.f[0], s.f[1], s.f[2], s.f[3]};
+                d.drift = (int32_t)(s.sk * es % 16);
+                if (!k.tma[tma % kTmaClasses].encode(d.maps, d.off, field, s.ni, s.nj, s.nk, s.sj, s.sk, d.wsh))
+                    encoded = false;
+            }
             d.items_i = (int32_t)ceil_div(s.ni, b->vadv_block);
             d.items_j = (int32_t)s.nj;
             items += (int64_t)d.items_i * d.items_j;
         }
     };
-    int64_t hitems = 0;
-    for (int q : hd) fill(q, hitems);
-    t->n_hdiff = (int32_t)hd.size();
-    t->hdiff_items = hitems;
-    int64_t total = hitems;
-    for (int bk = 0; bk < kBuckets; ++bk) {
-        t->bucket_first[bk] = slot;
-        int64_t items = 0;
-        for (int q : vd[bk]) fill(q, items);
-        t->bucket_items[bk] = items;
-        total += items;
+    int64_t total = 0;
+    auto fill_all = [&]() {
+        slot = 0;
+        int64_t hitems = 0;
+        for (int q : hd) fill(q, hitems);
+        t->n_hdiff = (int32_t)hd.size();
+        t->hdiff_items = hitems;
+        total = hitems;
+        if (tma >= 0) {  // one queue, tallest first
+            t->bucket_first[0] = slot;
+            int64_t items = 0;
+            for (int bk = kBuckets - 1; bk >= 0; --bk)
+                for (int q : vd[bk]) fill(q, items);
+            t->bucket_items[0] = items;
+            for (int bk = 1; bk < kBuckets; ++bk) {
+                t->bucket_first[bk] = slot;
+                t->bucket_items[bk] = 0;
+            }
+            total += items;
+            return;
+        }
+        for (int bk = 0; bk < kBuckets; ++bk) {
+            t->bucket_first[bk] = slot;
+            int64_t items = 0;
+            for (int q : vd[bk]) fill(q, items);
+            t->bucket_items[bk] = items;
+            total += items;
+        }
+    };
+    fill_all();
+    if (tma >= 0 && (!encoded || idx64)) {  // the driver refused a map, or an hdiff domain needs 64-bit offsets
+        tma = -1;
+        fill_all();
     }
     t->bucket_first[kBuckets] = slot;
     t->ndomains = n;
     b->total_items = total;
     b->idx64 = idx64;
     b->use_tmem = tmem_ok && !idx64;
+    b->use_tma = tma;
     return SB_OK;
 }
 
@@ -641,14 +927,20 @@ int sb_batch_launch(sb_batch* b, void* stream, double* time_s) {
     SB_CUDA(cudaGetDevice(&dev));
     SB_CHECK(dev == b->device, SB_ERR_INVALID, "batch was created on device %d, current device is %d", b->device,
              dev);
-    if (!b->exec || b->graph_idx64 != b->idx64 || b->graph_tmem != b->use_tmem) {
-        int rc = capture_graph(b);
+    // a give-up of an earlier launch is reported before anything new runs
+    int rc = take_wait_status();
+    if (rc) return rc;
+    if (!b->exec || b->graph_idx64 != b->idx64 || b->graph_tmem != b->use_tmem || b->graph_tma != b->use_tma ||
+        (b->use_tma >= 0 && b->graph_polls != wait_polls())) {
+        rc = capture_graph(b);
         if (rc) return rc;
     }
-    return timed((cudaStream_t)stream, time_s, [&]() {
+    rc = timed((cudaStream_t)stream, time_s, [&]() {
         SB_CUDA(cudaGraphLaunch(b->exec, (cudaStream_t)stream));
         return SB_OK;
     });
+    if (rc == SB_OK && time_s && b->use_tma >= 0) rc = take_wait_status();
+    return rc;
 }
 
 int sb_batch_info(sb_batch* b, int64_t* total_items, size_t* workspace_bytes, int* grid, int* block) {

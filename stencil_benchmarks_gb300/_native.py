@@ -243,6 +243,9 @@ def timed_out():
 
 
 def storage_code(dtype) -> int:
+    code = DTYPE_CODES.get(dtype) if isinstance(dtype, str) else None
+    if code is not None:
+        return code
     name = dtype if isinstance(dtype, str) else np.dtype(dtype).name
     try:
         return DTYPE_CODES[name]

@@ -77,11 +77,6 @@ template <class S, class C>
 constexpr int kBatchV = std::is_same<C, fix64>::value || (sizeof(S) != sizeof(C) && sizeof(S) == 4) ? 0
                         : sizeof(S) == 2                                                           ? 4
                                                                                                    : 2;
-// output columns of a strip
-template <class S, class C>
-constexpr int kBatchStep = kBatchV<S, C> == 0 ? kJscanOut
-                                              : 32 * kBatchV<S, C> - kBatchV<S, C> * ((4 + kBatchV<S, C> - 1) / (kBatchV<S, C> == 0 ? 1 : kBatchV<S, C>));
-
 // the domain of an item among [lo, hi]: the last one whose first item is not past it
 __device__ __forceinline__ int find_domain(const DevTable* __restrict__ tab, int lo, int hi, int64_t item) {
     while (lo < hi) {
@@ -116,11 +111,11 @@ __global__ void __launch_bounds__(256)
         const int j1 = min(dm.nj, j0 + rows);
         if constexpr (kBatchV<S, C> > 0) {
             if (dm.vec) {
-                constexpr int V = kBatchV<S, C>, step = kBatchStep<S, C>;
+                constexpr int V = kBatchV<S, C>;
                 for (int k = k0; k < k1; ++k)
-                    hdiff_vscan_strip<S, C, V, (V == 4 ? 1 : U), IDX>((const S*)dm.f[0], (const S*)dm.f[1], (S*)dm.out,
-                                                                      dm.ni, dm.nj, (IDX)dm.sj, (IDX)dm.sk,
-                                                                      dm.cs0 + strip * step, step, lane, j0, j1, k);
+                    hdiff_vscan_strip<S, C, V, (V == 4 ? 1 : U), IDX, true>(
+                        (const S*)dm.f[0], (const S*)dm.f[1], (S*)dm.out, dm.ni, dm.nj, (IDX)dm.sj, (IDX)dm.sk,
+                        dm.cs0 + strip * kStripStep<V, true>, lane, j0, j1, k);
                 continue;
             }
         }
@@ -418,7 +413,7 @@ Kinds kinds_for() {
     k.slab = SLAB;
     k.sift = std::is_same<S, double>::value && std::is_same<HC, double>::value;
     k.hdiff_v = k.sift ? 0 : kBatchV<S, HC>;
-    k.hdiff_step = kBatchStep<S, HC>;
+    k.hdiff_step = kBatchV<S, HC> == 4 ? kStripStep<4, true> : kStripStep<2, true>;
     if constexpr (std::is_same<S, double>::value && std::is_same<HC, double>::value)
         k.hdiff = [](dim3 g, dim3, cudaStream_t s, const DevTable* t, unsigned long long* c) {
             batch_sift_kernel<IDX><<<g, 32 * kSiftWarps, 0, s>>>(t, c);

@@ -172,39 +172,41 @@ int launch_jscan(const void* inp, const void* coeff, void* out, int64_t ni, int6
 // VSCAN: warp strips of 32*V columns (hdiff_vscan_strip), strip s = blockIdx.x
 // starting at column cs0 + s*step; the warps of a block take consecutive
 // TY-row tiles of that strip (few strips per domain, so no idle warps).
-template <class S, class C, int V, int U, class IDX>
+template <class S, class C, int V, int U, class IDX, bool VEC>
 __global__ void __launch_bounds__(256)
     hdiff_vscan_kernel(const S* __restrict__ inp, const S* __restrict__ coeff, S* __restrict__ out, int ni, int nj,
-                       int nk, IDX sj, IDX sk, int cs0, int step, int TY, int kper) {
-    const int strip = blockIdx.x;
+                       int nk, IDX sj, IDX sk, int cs0, int TY, int kper) {
     const int j0 = (blockIdx.y * blockDim.y + threadIdx.y) * TY;
     if (j0 >= nj) return;  // whole warp
     const int j1 = min(nj, j0 + TY);
     const int k0 = blockIdx.z * kper;
     const int k1 = min(nk, k0 + kper);
     for (int k = k0; k < k1; ++k)
-        hdiff_vscan_strip<S, C, V, U, IDX>(inp, coeff, out, ni, nj, sj, sk, cs0 + strip * step, step, threadIdx.x,
-                                           j0, j1, k);
+        hdiff_vscan_strip<S, C, V, U, IDX, VEC>(inp, coeff, out, ni, nj, sj, sk,
+                                                cs0 + (int)blockIdx.x * kStripStep<V, VEC>, threadIdx.x, j0, j1, k);
 }
 
-// VSCAN launch if the layout qualifies: i unit-stride, j/k strides multiples
-// of the vector size, and inp / coeff / out at the same offset from a vector
-// boundary (then one column grid is vector-aligned in all three fields);
-// SB_ERR_UNSUPPORTED (no error text) if not.
-template <class S, class C, int V>
+// VSCAN launch if the layout qualifies: i unit-stride and positive strides, and
+// for VEC j/k strides multiples of the vector size, and inp / coeff / out at
+// the same offset from a vector boundary (then one column grid is
+// vector-aligned in all three fields); SB_ERR_UNSUPPORTED (no error text) if not.
+template <class S, class C, int V, bool VEC>
 int launch_vscan(const void* inp, const void* coeff, void* out, int64_t ni, int64_t nj, int64_t nk, int64_t si,
                  int64_t sj, int64_t sk, int nw, int ty, int kper, int unroll, cudaStream_t stream,
                  const DeviceProps* p) {
     constexpr int ES = (int)sizeof(S), VB = V * ES;
-    if (si != 1 || sj <= 0 || sk <= 0 || (sj * ES) % VB || (sk * ES) % VB) return SB_ERR_UNSUPPORTED;
-    const uintptr_t a = (uintptr_t)inp;
-    if (a % ES || (uintptr_t)coeff % VB != a % VB || (uintptr_t)out % VB != a % VB) return SB_ERR_UNSUPPORTED;
+    if (si != 1 || sj <= 0 || sk <= 0) return SB_ERR_UNSUPPORTED;
+    int cs0 = -2;
+    if constexpr (VEC) {
+        if ((sj * ES) % VB || (sk * ES) % VB) return SB_ERR_UNSUPPORTED;
+        const uintptr_t a = (uintptr_t)inp;
+        if (a % ES || (uintptr_t)coeff % VB != a % VB || (uintptr_t)out % VB != a % VB) return SB_ERR_UNSUPPORTED;
+        const int off = (int)((a % VB) / ES);
+        cs0 = -2 - (((off - 2) % V) + V) % V;  // <= -2, (off + cs0) % V == 0
+    }
     SB_CHECK(nw >= 1 && nw <= 8, SB_ERR_INVALID, "vscan: 1..8 warps per block");
     SB_CHECK(ty >= 1 && kper >= 1, SB_ERR_INVALID, "vscan: tile_y and k_per_cta must be positive");
-    const int off = (int)((a % VB) / ES);
-    const int cs0 = -2 - (((off - 2) % V) + V) % V;  // <= -2, (off + cs0) % V == 0
-    const int step = 32 * V - V * ((4 + V - 1) / V);
-    const int64_t nstrips = ceil_div(ni - (cs0 + 2), (int64_t)step);
+    const int64_t nstrips = ceil_div(ni - (cs0 + 2), (int64_t)kStripStep<V, VEC>);
     const int64_t gx = nstrips, gy = ceil_div(ceil_div(nj, ty), (int64_t)nw), gz = ceil_div(nk, kper);
     SB_CHECK(gy <= p->max_grid_y && gz <= p->max_grid_z, SB_ERR_INVALID, "hdiff grid too large");
     const dim3 grid((unsigned)gx, (unsigned)gy, (unsigned)gz), block(32, nw);
@@ -212,9 +214,8 @@ int launch_vscan(const void* inp, const void* coeff, void* out, int64_t ni, int6
     const int64_t hi = ni + 2 + 32 * V + (nj + 2) * sj + nk * sk;
     const bool small = lo > -(1LL << 31) && hi < (1LL << 31);
 #define SB_VSCAN(UV, IDXT)                                                                                   \
-    hdiff_vscan_kernel<S, C, V, UV, IDXT><<<grid, block, 0, stream>>>(                                        \
-        (const S*)inp, (const S*)coeff, (S*)out, (int)ni, (int)nj, (int)nk, (IDXT)sj, (IDXT)sk, cs0, step,    \
-        ty, kper)
+    hdiff_vscan_kernel<S, C, V, UV, IDXT, VEC><<<grid, block, 0, stream>>>(                                   \
+        (const S*)inp, (const S*)coeff, (S*)out, (int)ni, (int)nj, (int)nk, (IDXT)sj, (IDXT)sk, cs0, ty, kper)
 #define SB_VSCAN_U(IDXT)                                                                                     \
     switch (unroll) {                                                                                         \
         case 1: SB_VSCAN(1, IDXT); break;                                                                     \
@@ -577,18 +578,33 @@ int launch_typed(const void* inp, const void* coeff, void* out, int64_t ni, int6
         }
     }
     // bfloat16 storage, float-pair and float32 compute: vector strips (V
-    // columns per lane) issue fewer instructions per point than JSCAN (56 vs
-    // 62 us, 271 vs 313 us and, with V = 2, 51 vs 53 us at 512x512x80).
+    // columns per lane, packed float32 arithmetic) issue fewer instructions per
+    // point than JSCAN (44 vs 62 us, 273 vs 313 us and, with V = 2, 46 vs 53 us at
+    // 512x512x80; 56 and 49 with scalar arithmetic and rows loaded U at a time).
     if constexpr (std::is_same<S, bf16>::value || std::is_same<C, f32x2>::value) {
         if (variant == SB_VARIANT_AUTO) {
             constexpr int V = sizeof(S) == 8 ? 2 : 4;
-            const int rc_v = launch_vscan<S, C, V>(inp, coeff, out, ni, nj, nk, si, sj, sk, 1, 16, 1, 1, stream, p);
+            const int rc_v = launch_vscan<S, C, V, true>(inp, coeff, out, ni, nj, nk, si, sj, sk, 1, 16, 1, 1, stream, p);
             if (rc_v != SB_ERR_UNSUPPORTED) return rc_v;
         }
     }
     if constexpr (std::is_same<S, float>::value && std::is_same<C, float>::value) {
         if (variant == SB_VARIANT_AUTO) {
-            const int rc_v = launch_vscan<S, C, 2>(inp, coeff, out, ni, nj, nk, si, sj, sk, 2, 16, 1, 4, stream, p);
+            const int rc_v = launch_vscan<S, C, 2, true>(inp, coeff, out, ni, nj, nk, si, sj, sk, 2, 16, 1, 4, stream, p);
+            if (rc_v != SB_ERR_UNSUPPORTED) return rc_v;
+        }
+    }
+    // Rows that no aligned vectors fit (odd strides, fields at different offsets):
+    // the same strips with single elements, two columns per lane; JSCAN strips
+    // spend 76 instructions per point where these spend about 35.  391x263x97:
+    // bfloat16 27.0 us (JSCAN 38.2), float32 28.6 (31.1), float pair 148 (175);
+    // 1001x61x100 bfloat16 18.3 (22.2), float32 18.9 (18.9); 513x511x80 47 (60) and
+    // 51.6 (50.7).
+    if constexpr (!std::is_same<C, fix64>::value && !std::is_same<C, double>::value) {
+        if (variant == SB_VARIANT_AUTO) {
+            constexpr bool f32 = std::is_same<S, float>::value, pairs = std::is_same<C, f32x2>::value;
+            const int rc_v = launch_vscan<S, C, 2, false>(inp, coeff, out, ni, nj, nk, si, sj, sk, f32 ? 2 : 1, f32 ? 8 : 16,
+                                                          1, pairs ? 1 : 4, stream, p);
             if (rc_v != SB_ERR_UNSUPPORTED) return rc_v;
         }
     }
@@ -639,20 +655,20 @@ int launch_typed(const void* inp, const void* coeff, void* out, int64_t ni, int6
             if constexpr (sizeof(S) == 8) {
                 if (width == 64) {
                     shape_ok = true;
-                    rc2 = launch_vscan<S, C, 2>(inp, coeff, out, ni, nj, nk, si, sj, sk, nw, ty, kper, unroll, stream, p);
+                    rc2 = launch_vscan<S, C, 2, true>(inp, coeff, out, ni, nj, nk, si, sj, sk, nw, ty, kper, unroll, stream, p);
                 }
             } else if constexpr (sizeof(S) == 4) {
                 if (width == 64 || width == 128) shape_ok = true;
                 if (width == 64)
-                    rc2 = launch_vscan<S, C, 2>(inp, coeff, out, ni, nj, nk, si, sj, sk, nw, ty, kper, unroll, stream, p);
+                    rc2 = launch_vscan<S, C, 2, true>(inp, coeff, out, ni, nj, nk, si, sj, sk, nw, ty, kper, unroll, stream, p);
                 if (width == 128)
-                    rc2 = launch_vscan<S, C, 4>(inp, coeff, out, ni, nj, nk, si, sj, sk, nw, ty, kper, unroll, stream, p);
+                    rc2 = launch_vscan<S, C, 4, true>(inp, coeff, out, ni, nj, nk, si, sj, sk, nw, ty, kper, unroll, stream, p);
             } else {
                 if (width == 128 || width == 256) shape_ok = true;
                 if (width == 128)
-                    rc2 = launch_vscan<S, C, 4>(inp, coeff, out, ni, nj, nk, si, sj, sk, nw, ty, kper, unroll, stream, p);
+                    rc2 = launch_vscan<S, C, 4, true>(inp, coeff, out, ni, nj, nk, si, sj, sk, nw, ty, kper, unroll, stream, p);
                 if (width == 256)
-                    rc2 = launch_vscan<S, C, 8>(inp, coeff, out, ni, nj, nk, si, sj, sk, nw, ty, kper, unroll, stream, p);
+                    rc2 = launch_vscan<S, C, 8, true>(inp, coeff, out, ni, nj, nk, si, sj, sk, nw, ty, kper, unroll, stream, p);
             }
             SB_CHECK(shape_ok, SB_ERR_INVALID,
                      "hdiff vscan strip width (block_x) must be 64 for 8-byte, 64 or 128 for 4-byte and 128 or 256 "

@@ -97,9 +97,104 @@ __device__ __forceinline__ void hdiff_jscan_strip(const S* __restrict__ inp, con
 // ---------------------------------------------------------------------------
 // horizontal diffusion, one warp, one k-plane strip of 32*V columns
 // ---------------------------------------------------------------------------
+// Two neighbouring columns of one row.  float32 pairs use the packed
+// instructions, one per two rounded operations (14.9 against 10.4 T pairs/s for
+// two scalar additions); the rounding of each half is the scalar one's.
+template <class C>
+struct Pair {
+    C a, b;
+};
+template <class C>
+__device__ __forceinline__ Pair<C> pair_add(Pair<C> p, Pair<C> q) {
+    return {Ar<C>::add(p.a, q.a), Ar<C>::add(p.b, q.b)};
+}
+template <class C>
+__device__ __forceinline__ Pair<C> pair_sub(Pair<C> p, Pair<C> q) {
+    return {Ar<C>::sub(p.a, q.a), Ar<C>::sub(p.b, q.b)};
+}
+template <class C>
+__device__ __forceinline__ Pair<C> pair_mul(Pair<C> p, Pair<C> q) {
+    return {Ar<C>::mul(p.a, q.a), Ar<C>::mul(p.b, q.b)};
+}
+template <class C>
+__device__ __forceinline__ Pair<C> pair_times4(Pair<C> p) {
+    return {Ar<C>::template scale2<2>(p.a), Ar<C>::template scale2<2>(p.b)};
+}
+template <class C>
+__device__ __forceinline__ Pair<C> pair_limit(Pair<C> f, Pair<C> x1, Pair<C> x0) {
+    return {Ar<C>::limit(f.a, x1.a, x0.a), Ar<C>::limit(f.b, x1.b, x0.b)};
+}
+// Products whose sign alone matters.  The products that are subtracted from
+// something stay scalar (pair_mul, pair_times4): a packed product and the
+// subtraction after it can be fused by the assembler, which rounds once.
+template <class C>
+__device__ __forceinline__ Pair<C> pair_sign_product(Pair<C> p, Pair<C> q) {
+    return pair_mul<C>(p, q);
+}
+#define SB_PAIR_OP(NAME, INSTR)                                                                                  \
+    template <>                                                                                                  \
+    __device__ __forceinline__ Pair<float> NAME<float>(Pair<float> p, Pair<float> q) {                           \
+        Pair<float> r;                                                                                           \
+        asm("{\n .reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n " INSTR                       \
+            " z, x, y;\n mov.b64 {%0, %1}, z;\n}\n"                                                              \
+            : "=f"(r.a), "=f"(r.b)                                                                               \
+            : "f"(p.a), "f"(p.b), "f"(q.a), "f"(q.b));                                                           \
+        return r;                                                                                                \
+    }
+SB_PAIR_OP(pair_add, "add.rn.f32x2")
+SB_PAIR_OP(pair_sub, "sub.rn.f32x2")
+SB_PAIR_OP(pair_sign_product, "mul.rn.f32x2")
+#undef SB_PAIR_OP
+template <>
+__device__ __forceinline__ Pair<float> pair_limit<float>(Pair<float> f, Pair<float> x1, Pair<float> x0) {
+    const Pair<float> m = pair_sign_product<float>(f, pair_sub<float>(x1, x0));
+    return {m.a > 0.0f ? 0.0f : f.a, m.b > 0.0f ? 0.0f : f.b};
+}
+
+// V storage elements as they come from memory, converted when they are used, so
+// that a row can be loaded rows ahead of its use: one vector, or V elements of
+// which those not in `one` are zero.
+template <class S, int V, bool VEC>
+struct RowPiece {
+    typename RawVec<(int)sizeof(S) * V>::T r;
+    __device__ __forceinline__ void load(const S* __restrict__ p, bool group, const bool (&)[V]) {
+        r = {};
+        if (group) r = __ldg(reinterpret_cast<const decltype(r)*>(p));
+    }
+    template <class C>
+    __device__ __forceinline__ void get(Pair<C> (&p)[V / 2]) const {
+        S e[V];
+        memcpy(e, &r, sizeof(r));
+#pragma unroll
+        for (int n = 0; n < V / 2; ++n) p[n] = {cvt<C, S>(e[2 * n]), cvt<C, S>(e[2 * n + 1])};
+    }
+};
+template <class S, int V>
+struct RowPiece<S, V, false> {
+    S e[V];
+    __device__ __forceinline__ void load(const S* __restrict__ p, bool group, const bool (&one)[V]) {
+#pragma unroll
+        for (int q = 0; q < V; ++q) {
+            e[q] = S(0.0f);
+            if (group && one[q]) e[q] = __ldg(p + q);
+        }
+    }
+    template <class C>
+    __device__ __forceinline__ void get(Pair<C> (&p)[V / 2]) const {
+#pragma unroll
+        for (int n = 0; n < V / 2; ++n) p[n] = {cvt<C, S>(e[2 * n]), cvt<C, S>(e[2 * n + 1])};
+    }
+};
+
+// output columns of a strip: with vectors the first column of a strip lies on a
+// vector boundary, so strips advance by whole vectors
+template <int V, bool VEC>
+constexpr int kStripStep = VEC ? 32 * V - V * ((4 + V - 1) / V) : 32 * V - 4;
+
 // The JSCAN march with V columns per lane: lane L holds columns
-// c = cs + V*L + q (q < V) of each row, moved as one aligned vector of
-// V*sizeof(S) bytes (the caller picks cs so that column cs starts a vector).
+// c = cs + V*L + q (q < V) of each row.  VEC: they are moved as one aligned
+// vector of V*sizeof(S) bytes (the caller picks cs so that column cs starts a
+// vector); else element by element, at any alignment and row stride.
 // Neighbours inside a lane's group are registers; across lanes four shuffles
 // per row serve V points (inp left/right, lap right, flx left).  Outputs are
 // the columns [cs+2, cs+2+step) within [0, ni).  A vector is loaded when it
@@ -107,102 +202,125 @@ __device__ __forceinline__ void hdiff_jscan_strip(const S* __restrict__ inp, con
 // lie in the same aligned V*sizeof(S)-byte block of the caller's memory and
 // only feed points that are not stored.  Same arithmetic and order as
 // hdiff_jscan_strip.  All 32 lanes must call this (full-mask shuffles).
-template <class S, class C, int V, int U, class IDX>
+template <class S, class C, int V, int U, class IDX, bool VEC>
 __device__ __forceinline__ void hdiff_vscan_strip(const S* __restrict__ inp, const S* __restrict__ coeff,
                                                   S* __restrict__ out, int ni, int nj, IDX sj, IDX sk, int cs,
-                                                  int step, int lane, int j0, int j1, int k) {
-    using A = Ar<C>;
+                                                  int lane, int j0, int j1, int k) {
+    constexpr int step = kStripStep<V, VEC>, NP = V / 2;
+    using PC = Pair<C>;
     const int c0 = cs + V * lane;
-    const bool grp_in = c0 + V > -2 && c0 < ni + 2;
     const int wlo = max(cs + 2, 0), whi = min(cs + 2 + step, ni);
     const bool any_w = c0 + V > wlo && c0 < whi;
     const bool all_w = c0 >= wlo && c0 + V <= whi;
-    const int rmax = nj + 1;
-    const IDX obase = (IDX)k * sk + (IDX)c0;
-    auto load_row = [&](int r, C(&o)[V]) {
-        if (grp_in && r <= rmax) {
-            ld_vec<S, C, V>(inp + (obase + (IDX)r * sj), o);
-        } else {
+    const bool grp_in = c0 + V > -2 && c0 < ni + 2;
+    bool in[V], w[V];
 #pragma unroll
-            for (int q = 0; q < V; ++q) o[q] = C(0);
+    for (int q = 0; q < V; ++q) {
+        in[q] = c0 + q >= -2 && c0 + q < ni + 2;
+        w[q] = c0 + q >= wlo && c0 + q < whi;
+    }
+    IDX at = (IDX)k * sk + (IDX)c0 + (IDX)j0 * sj;  // this lane's first column in output row j0
+    using Row = RowPiece<S, V, VEC>;
+    // Rows j + 2 of inp and j of coeff of U output rows.  Two-byte storage: always
+    // the next U rows in flight, each reloaded when used (512x512x80 bfloat16
+    // 44 us, 49 loading U at a time).  Wider storage: U rows loaded together, then
+    // computed (float32 48 us, 52 with the rows always in flight, whose separate
+    // waits outnumber the hardware's scoreboards).
+    constexpr bool RING = sizeof(S) == 2;
+    Row rin[U], rcf[U];
+    auto load_rows = [&](int j) {  // of output rows j .. j + U - 1
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const bool row = j + u < j1;  // then row j + u + 2 <= nj + 1 exists
+            rin[u].load(inp + (at + (IDX)(u + 2) * sj), row && grp_in, in);
+            rcf[u].load(coeff + (at + (IDX)u * sj), row && any_w, w);
         }
     };
-    // lap of the centre row c given the rows below (b) and above (a)
-    auto lap_row = [&](const C(&b)[V], const C(&c)[V], const C(&a)[V], C(&o)[V], C& right) {
-        const C left = shfl_up(c[V - 1], 1);  // column c0 - 1
-        right = shfl_down(c[0], 1);           // column c0 + V
+    if (RING) load_rows(j0);
+    // lap of the centre row c given the rows below (b) and above (a); right: column c0 + V of c
+    auto lap_row = [&](const PC(&b)[NP], const PC(&c)[NP], const PC(&a)[NP], PC(&o)[NP], C& right) {
+        const C left = shfl_up(c[NP - 1].b, 1);  // column c0 - 1
+        right = shfl_down(c[0].a, 1);
 #pragma unroll
-        for (int q = 0; q < V; ++q) {
-            const C l = q == 0 ? left : c[q - 1];
-            const C r = q == V - 1 ? right : c[q + 1];
-            o[q] = A::sub(A::template scale2<2>(c[q]), A::add(A::add(A::add(r, l), a[q]), b[q]));
+        for (int n = 0; n < NP; ++n) {
+            const PC l = {n == 0 ? left : c[n - 1].b, c[n].a};
+            const PC r = {c[n].b, n == NP - 1 ? right : c[n + 1].a};
+            o[n] = pair_sub<C>(pair_times4<C>(c[n]), pair_add<C>(pair_add<C>(pair_add<C>(r, l), a[n]), b[n]));
         }
     };
-    C am2[V], a0[V], a1[V], a2[V], lap_m1[V], lap0[V], fly_m1[V];
-    load_row(j0 - 2, am2);
-    load_row(j0 - 1, a0);
-    load_row(j0, a1);
-    load_row(j0 + 1, a2);
+    PC am2[NP], a0[NP], a1[NP], a2[NP], lap_m1[NP], lap0[NP], fly_m1[NP];
+    {
+        Row r[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) r[t].load(inp + (at + (IDX)(t - 2) * sj), grp_in, in);
+        r[0].get(am2);
+        r[1].get(a0);
+        r[2].get(a1);
+        r[3].get(a2);
+    }
     C unused, rnb0;
     lap_row(am2, a0, a1, lap_m1, unused);  // lap(j0-1)
     lap_row(a0, a1, a2, lap0, rnb0);       // lap(j0); rnb0 = inp(c0+V, j0)
 #pragma unroll
-    for (int q = 0; q < V; ++q) {
-        fly_m1[q] = A::limit(A::sub(lap0[q], lap_m1[q]), a1[q], a0[q]);  // fly(j0-1)
-        a0[q] = a1[q];
-        a1[q] = a2[q];
+    for (int n = 0; n < NP; ++n) {
+        fly_m1[n] = pair_limit<C>(pair_sub<C>(lap0[n], lap_m1[n]), a1[n], a0[n]);  // fly(j0-1)
+        a0[n] = a1[n];
+        a1[n] = a2[n];
     }
     // state for output row j: a0 = inp(j), a1 = inp(j+1), lap0 = lap(j), rnb0 = inp(c0+V, j)
     for (int jb = j0; jb < j1; jb += U) {
-        C nxt[U][V], cf[U][V];
+        if (!RING) load_rows(jb);
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            const int j = jb + u;
-            load_row(j + 2, nxt[u]);
-            if (any_w && j < j1) {
-                ld_vec<S, C, V>(coeff + (obase + (IDX)j * sj), cf[u]);
-            } else {
-#pragma unroll
-                for (int q = 0; q < V; ++q) cf[u][q] = C(0);
+            if (U > 1 && jb + u >= j1) break;  // warp-uniform
+            PC nxt[NP], cf[NP], lap1[NP], fly0[NP], flx0[NP], res[NP];
+            rin[u].get(nxt);
+            rcf[u].get(cf);
+            if (RING) {
+                const bool row = jb + u + U < j1;
+                rin[u].load(inp + (at + (IDX)(U + 2) * sj), row && grp_in, in);
+                rcf[u].load(coeff + (at + (IDX)U * sj), row && any_w, w);
             }
-        }
+            C rnb1;
+            lap_row(a0, a1, nxt, lap1, rnb1);
+            const C lapR = shfl_down(lap0[0].a, 1);  // lap(c0+V, j)
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int j = jb + u;
-            if (j >= j1) break;  // warp-uniform
-            C lap1[V], fly0[V], flx0[V], res[V], rnb1;
-            lap_row(a0, a1, nxt[u], lap1, rnb1);
-            const C lapR = shfl_down(lap0[0], 1);  // lap(c0+V, j)
-#pragma unroll
-            for (int q = 0; q < V; ++q) {
-                fly0[q] = A::limit(A::sub(lap1[q], lap0[q]), a1[q], a0[q]);
-                const C lr = q == V - 1 ? lapR : lap0[q + 1];
-                const C ir = q == V - 1 ? rnb0 : a0[q + 1];
-                flx0[q] = A::limit(A::sub(lr, lap0[q]), ir, a0[q]);
+            for (int n = 0; n < NP; ++n) {
+                fly0[n] = pair_limit<C>(pair_sub<C>(lap1[n], lap0[n]), a1[n], a0[n]);
+                const PC lr = {lap0[n].b, n == NP - 1 ? lapR : lap0[n + 1].a};
+                const PC ir = {a0[n].b, n == NP - 1 ? rnb0 : a0[n + 1].a};
+                flx0[n] = pair_limit<C>(pair_sub<C>(lr, lap0[n]), ir, a0[n]);
             }
-            const C flxL = shfl_up(flx0[V - 1], 1);  // flx(c0-1, j)
+            const C flxL = shfl_up(flx0[NP - 1].b, 1);  // flx(c0-1, j)
 #pragma unroll
-            for (int q = 0; q < V; ++q) {
-                const C fl = q == 0 ? flxL : flx0[q - 1];
-                const C d = A::sub(A::add(A::sub(flx0[q], fl), fly0[q]), fly_m1[q]);
-                res[q] = A::sub(a0[q], A::mul(cf[u][q], d));
+            for (int n = 0; n < NP; ++n) {
+                const PC fl = {n == 0 ? flxL : flx0[n - 1].b, flx0[n].a};
+                const PC d = pair_sub<C>(pair_add<C>(pair_sub<C>(flx0[n], fl), fly0[n]), fly_m1[n]);
+                res[n] = pair_sub<C>(a0[n], pair_mul<C>(cf[n], d));
             }
-            S* orow = out + (obase + (IDX)j * sj);
-            if (all_w) {
-                st_vec<S, C, V>(orow, res);
+            S* orow = out + at;
+            C v[V];
+#pragma unroll
+            for (int n = 0; n < NP; ++n) {
+                v[2 * n] = res[n].a;
+                v[2 * n + 1] = res[n].b;
+            }
+            if (VEC && all_w) {
+                if constexpr (VEC) st_vec<S, C, V>(orow, v);
             } else if (any_w) {
 #pragma unroll
                 for (int q = 0; q < V; ++q)
-                    if (c0 + q >= wlo && c0 + q < whi) st<S, C>(orow + q, res[q]);
+                    if (w[q]) st<S, C>(orow + q, v[q]);
             }
 #pragma unroll
-            for (int q = 0; q < V; ++q) {
-                a0[q] = a1[q];
-                a1[q] = nxt[u][q];
-                lap0[q] = lap1[q];
-                fly_m1[q] = fly0[q];
+            for (int n = 0; n < NP; ++n) {
+                a0[n] = a1[n];
+                a1[n] = nxt[n];
+                lap0[n] = lap1[n];
+                fly_m1[n] = fly0[n];
             }
             rnb0 = rnb1;
+            at += sj;
         }
     }
 }

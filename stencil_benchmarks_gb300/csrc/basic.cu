@@ -144,11 +144,17 @@ __global__ void __launch_bounds__(256) lap_march_kernel(const S* __restrict__ in
     }
 }
 
-// float64 placements of the along-x-and-y strips (sites 0-4), by preset: 1 all
-// fp64, 2 the closing addition, 3 the second subtraction of each axis, 4 both
-// of those and the addition (0 selects the default preset)
+// float64 placements (sites of lap_march_kernel).  The default moves the second
+// subtraction of each axis to the integer pipe; presets of the along-x-and-y
+// strips: 1 all fp64, 2 the closing addition, 3 the second subtraction of each
+// axis (the default), 4 those and the addition; other axis sets take the
+// default or, with a preset, run all fp64.  512x512x80 along x and y, five
+// operations per point: all on the fp64 pipe 247 us, one on the integer pipe
+// 207, two 187, three 262 (an fp64 operation takes about 41 us of that pipe, an
+// integer one 70 us of the ALU pipe); along one axis 103-108 against 126, along
+// three 297 against 366.
+constexpr uint32_t kLapDefaultSites = 0x4Au;
 constexpr uint32_t kLapPlacements[] = {0u, 0u, 0x10u, 0x0Au, 0x1Au};
-constexpr int kLapPlacementDefault = 1;
 
 template <int MASK, class S, class C, int R, int PK>
 int launch_lap_march_pl(int placement, const S* inp, S* out, int64_t ni, int64_t nj, int64_t nk, int64_t si,
@@ -160,6 +166,8 @@ int launch_lap_march_pl(int placement, const S* inp, S* out, int64_t ni, int64_t
         kernel<<<grid, block, 0, stream>>>(inp, out, (int)ni, (int)nj, (int)nk, si, sj, sk);
         return SB_OK;
     };
+    if constexpr (std::is_same<C, double>::value)
+        if (placement == 0) return go(lap_march_kernel<MASK, S, C, R, PK, kLapDefaultSites>);
     if constexpr (MASK == 3 && std::is_same<C, double>::value) {
         switch (placement) {
             case 2: return go(lap_march_kernel<MASK, S, C, R, PK, kLapPlacements[2]>);
@@ -199,7 +207,7 @@ int launch_lap_march(const void* inp, void* out, int64_t ni, int64_t nj, int64_t
              SB_ERR_INVALID, "domain too large for the Laplacian strip grid");
     const S* in = (const S*)inp;
     S* o = (S*)out;
-    const int pl = placement == 0 ? kLapPlacementDefault : placement;
+    const int pl = placement;
     switch (mask) {
 #define SB_LAP_MASK(M) \
     case M: return launch_lap_march_shape<M, S, C>(rows, pk, pl, in, o, ni, nj, nk, si, sj, sk, warps, stream);

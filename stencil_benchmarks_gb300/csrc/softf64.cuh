@@ -109,34 +109,34 @@ SB_SF_HD uint64_t round_pack(uint64_t sign, uint32_t e, uint64_t w) {
 // must compute it: a NaN or infinite operand, or a result below the normal
 // range (subnormal) or at or above 2^1024 before rounding.
 SB_SF_HD bool add(uint64_t a, uint64_t b, uint64_t& r) {
-    uint64_t ma = a & kAbs, mb = b & kAbs;
-    if (ma < mb) {
-        const uint64_t t = a, tm = ma;
-        a = b;
-        ma = mb;
-        b = t;
-        mb = tm;
-    }
-    const uint32_t ea = (uint32_t)(ma >> 52), eb = (uint32_t)(mb >> 52);
-    if (ea == 0x7ffu) return false;
-    const uint64_t fa = (ma & kMant) | ((uint64_t)(ea != 0u) << 52);
-    const uint64_t fb = (mb & kMant) | ((uint64_t)(eb != 0u) << 52);
-    const uint32_t ea1 = ea + (ea == 0u), eb1 = eb + (eb == 0u);
-    uint32_t d = ea1 - eb1;
+    // Order by magnitude, word by word: as a 64-bit compare and swap the compiler
+    // makes it minima and maxima that occupy the fp64 pipe (an addition beside an
+    // fp64 addition each: 246 G/s of both, 282 in this form).
+    const uint32_t ah = (uint32_t)(a >> 32), bh = (uint32_t)(b >> 32), al = (uint32_t)a, bl = (uint32_t)b;
+    const uint32_t ma = ah & 0x7fffffffu, mb = bh & 0x7fffffffu;
+    const bool swap = ma < mb || (ma == mb && al < bl);
+    const uint32_t xh = swap ? bh : ah, xl = swap ? bl : al, yh = swap ? ah : bh, yl = swap ? al : bl;
+    const uint32_t ex = (xh >> 20) & 0x7ffu, ey = (yh >> 20) & 0x7ffu;
+    if (ex == 0x7ffu) return false;
+    const uint64_t sign = (uint64_t)(xh & 0x80000000u) << 32;
+    const uint64_t fx = ((uint64_t)((xh & 0xfffffu) | (ex != 0u ? 0x100000u : 0u)) << 32) | xl;
+    const uint64_t fy = ((uint64_t)((yh & 0xfffffu) | (ey != 0u ? 0x100000u : 0u)) << 32) | yl;
+    const uint32_t ex1 = ex + (ex == 0u), ey1 = ey + (ey == 0u);
+    uint32_t d = ex1 - ey1;
     d = d > 63u ? 63u : d;
-    const uint64_t xa = fa << 10, xb = fb << 10;
-    uint64_t yb = xb >> d;
-    yb |= (uint64_t)((yb << d) != xb);
-    const bool sub = (int64_t)(a ^ b) < 0;
-    uint64_t s = sub ? xa - yb : xa + yb;
+    const uint64_t xs = fx << 10, ys = fy << 10;
+    uint64_t yb = ys >> d;
+    yb |= (uint64_t)((yb << d) != ys);
+    const bool diff = (int32_t)(xh ^ yh) < 0;
+    const uint64_t s = diff ? xs - yb : xs + yb;
     if (s == 0) {
-        r = sub ? 0ull : (a & kSign);  // exact cancellation gives +0; equal-signed zeros keep the sign
+        r = diff ? 0ull : sign;  // exact cancellation gives +0; equal-signed zeros keep the sign
         return true;
     }
     const int lz = clz64(s);
-    const int e = (int)ea1 - lz;
+    const int e = (int)ex1 - lz;
     if ((unsigned)e > 2045u) return false;
-    r = round_pack<11>(a & kSign, (uint32_t)e, s << lz);
+    r = round_pack<11>(sign, (uint32_t)e, s << lz);
     return true;
 }
 

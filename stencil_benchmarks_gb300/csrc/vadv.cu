@@ -96,7 +96,7 @@ constexpr uint32_t kVadvPlacements[] = {
     vadv_sites({4, 5, 7, 14, 16, 17, 20}) | kVadvRcpSite,
     vadv_sites({5, 7, 14, 17, 20}) | kVadvRcpSite,
 };
-static_assert(kVadvDefaultIntSites == (kVadvMuls | kVadvRcpSite), "the default split");
+static_assert(kVadvDefaultIntSites == ((kVadvMuls | kVadvRcpSite) & ~vadv_sites({13})), "the default split");
 // Measured at 512x512x80 (32-thread SLAB blocks): every site on the fp64
 // pipe 1171-1201 us whatever the blocks per SM or ring depth.  Depth 4, 24
 // blocks per SM: the nine products on the integer pipe (preset 2) 980-989 us
@@ -114,9 +114,12 @@ static_assert(kVadvDefaultIntSites == (kVadvMuls | kVadvRcpSite), "the default s
 // solved) is faster again: 742 us against 779 at depth 2, same bits.  The
 // default float64 SLAB form: depth 1, up to 28 blocks per SM, the grid
 // balanced so that every block takes the same number of groups.  (Figures from
-// before the negations left the fp64 pipe, see Ar<double>::neg: the default
-// runs in 662 us since, with that pipe 63%, the ALU pipe 55% and the issue
-// slots 62% busy.)
+// before the negations left the fp64 pipe, see Ar<double>::neg.  Since then all
+// nine + reciprocal run in 662 us, with that pipe 63%, the ALU pipe 55% and the
+// issue slots 62% busy, and one product fewer on the integer pipe is better:
+// without site 13 629 us (the default, preset 9), 4 631, 11 642, 16 634, 17 639,
+// 20 645; without two of them 631-684, without three 701; with an addition more,
+// 729-838.)
 constexpr int kVadvPlacementDefault = 9;
 constexpr int kVadvSlabBlocksPerSm = 28;
 constexpr int kVadvPlacementCount = (int)(sizeof(kVadvPlacements) / sizeof(kVadvPlacements[0]));

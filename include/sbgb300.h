@@ -301,7 +301,7 @@ typedef struct sb_domain {
 typedef struct sb_batch_tune {
     int32_t block;         /* threads per block, multiple of 32, <= 256 (0: 128)   */
     int32_t blocks_per_sm; /* persistent hdiff blocks per SM (0: 8; exact float64: 12) */
-    int32_t hdiff_rows;    /* rows of j per hdiff item (0: 32; exact float64: 16)  */
+    int32_t hdiff_rows;    /* rows of j per hdiff item (0: 32; exact float64: 20)  */
     int32_t hdiff_planes;  /* k-planes per hdiff item (0: 1)                       */
     int32_t order;         /* 0: the hdiff kernel enters the graph first; 1: the vadv
                             * bucket kernels first (tallest bucket first), so their

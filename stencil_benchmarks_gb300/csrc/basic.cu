@@ -27,7 +27,8 @@ template <class C>
 __device__ __forceinline__ C plus_zero(C t);
 template <>
 __device__ __forceinline__ double plus_zero<double>(double t) {
-    return ((__double_as_longlong(t) << 1) == 0) ? 0.0 : t;
+    // the zero test on the two words: on the whole pattern it becomes an fp64 instruction
+    return (((unsigned)__double2hiint(t) << 1) | (unsigned)__double2loint(t)) == 0u ? 0.0 : t;
 }
 template <>
 __device__ __forceinline__ float plus_zero<float>(float t) {

@@ -15,7 +15,7 @@
 //   hdiff_vscan_strip where the rows take aligned vectors, else
 //   hdiff_jscan_strip).  A warp takes the next item with one atomicAdd and
 //   finds its domain by binary search over the first-item offsets.  Exact
-//   float64: blocks take 60 x 16 tiles x `planes` planes (hdiff_sift.cuh).
+//   float64: blocks take 60 x 20 tiles x `planes` planes (hdiff_sift.cuh).
 // vadv: persistent blocks of BT threads; an item is BT consecutive columns of
 //   one j-row of one domain, one column per thread (stencil_core.cuh:
 //   vadv_async_column: cp.async-staged inputs).  Factors live in shared memory
@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-// Exact float64: blocks take 60 x 16 tiles (hdiff_sift.cuh).
+// Exact float64: blocks take 60 x 20 tiles (hdiff_sift.cuh).
 template <class IDX>
 __global__ void __launch_bounds__(32 * kSiftWarps, 9)
     batch_sift_kernel(const DevTable* __restrict__ tab, unsigned long long* __restrict__ counter) {

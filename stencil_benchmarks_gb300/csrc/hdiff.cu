@@ -234,7 +234,7 @@ int launch_vscan(const void* inp, const void* coeff, void* out, int64_t ni, int6
     return SB_OK;
 }
 
-// SIFT: one block per tile of 60 x 16 outputs of one plane (hdiff_sift.cuh).
+// SIFT: one block per tile of 60 x 20 outputs of one plane (hdiff_sift.cuh).
 template <class IDX>
 __global__ void __launch_bounds__(32 * kSiftWarps, 9)
     hdiff_sift_kernel(const double* __restrict__ inp, const double* __restrict__ coeff, double* __restrict__ out, int ni,
@@ -552,7 +552,7 @@ int launch_typed(const void* inp, const void* coeff, void* out, int64_t ni, int6
     int variant = tune ? tune->variant : SB_VARIANT_AUTO;
     const int placement = tune ? (tune->flags >> 4) & 15 : 0;
     // fp64 compute is bound by the fp64 pipe.  With float64 storage SIFT leaves
-    // out what the limiter zeroes (195 us at 512x512x80, figures and worst case
+    // out what the limiter zeroes (189 us at 512x512x80, figures and worst case
     // in hdiff_sift.cuh).  Otherwise TILE computes every lap/flx/fly once per
     // tile (fewest fp64 operations); fp32 and float-pair compute are
     // bound by instruction issue: JSCAN (shuffles, no block barriers) is faster.

@@ -33,9 +33,9 @@
 // a -0, a coefficient that is not finite, or more than kSiftCap open fluxes (a
 // quarter) are computed in full (hdiff_dense_tile).
 //
-// 512x512x80, U[0, 1): 195 us against 547 for the TMA tile, which computes
+// 512x512x80, U[0, 1): 189 us against 547 for the TMA tile, which computes
 // everything; 3.1 fp64 instructions per point instead of 11.6, that pipe 54% and
-// the issue slots 58% busy.  128x128x64: 19.3 us against 36.7.  On other fields,
+// the issue slots 58% busy.  128x128x64: 18.9 us against 36.7.  On other fields,
 // 512x512x40, against the tile's 278 us: 105 on U[0, 1) and U[-1, 1), 91 on a
 // smooth field, 124 to 227 on a ramp or a smooth field with noise, 293 where
 // half the fluxes pass and every tile is computed in full after all.
@@ -45,11 +45,15 @@
 
 namespace sb {
 
-constexpr int kSiftWarps = 4;                 // warps per tile (512x512x80: 1 warp 254 us, 2 198, 3 194, 4 195; 128x128x64: 22.0, 21.3, 19.8, 19.3)
-constexpr int kSiftRows = 16;                 // output rows of a tile
+// Warps and rows of a tile, 512x512x80 / 128x128x64 in us: 1, 2, 3, 4 warps on 16
+// rows 254 / 22.0, 198 / 21.3, 194 / 18.9, 195 / 18.7; 4 warps on 20, 24, 30 rows
+// 189 / 18.9, 191 / 19.0, 202 / 20.8; 8 warps on 31 rows 226 / 22.7.  Longer tiles
+// read fewer rows twice, but fewer of them fit an SM.
+constexpr int kSiftWarps = 4;
+constexpr int kSiftRows = 20;                 // output rows of a tile
 constexpr int kSiftCols = 64, kSiftOut = 60;  // columns read and written
 constexpr int kSiftSure = 17;                 // units beyond which a fixed-point flux has a certain sign
-constexpr int kSiftCap = 512;                 // open fluxes of a tile at most
+constexpr int kSiftCap = 640;                 // open fluxes of a tile at most
 
 struct SiftTile {
     double x[(kSiftRows + 4) * kSiftCols];  // row t: j0 - 2 + t, column c: cs + c
@@ -57,7 +61,7 @@ struct SiftTile {
     alignas(16) uint32_t open[(kSiftRows + 1) * 4];    // per row j0 - 1 + r: open flx of even / odd columns, open fly of even / odd
     uint16_t first[(kSiftRows + 1) * 4];   // where each of these masks' fluxes start in flux[]
     uint16_t list[kSiftRows * kSiftOut];   // open fluxes (row * 128 + direction * 64 + column), later points (row * 64 + column)
-    unsigned emax[4];                      // per warp: largest exponent field, 2^32 - 1 where the tile must be computed in full
+    unsigned emax[kSiftWarps];             // per warp: largest exponent field, 2^32 - 1 where the tile must be computed in full
 };
 
 // x as an integer multiple of 2^(E-1049), truncated toward zero (E: the largest
@@ -133,7 +137,7 @@ __device__ __noinline__ void hdiff_dense_tile(const double* tile, const double* 
     }
 }
 
-// The NW warps of a block, columns [cs + 2, cs + 62) and rows [j0, j0 + 16) of plane k.
+// The NW warps of a block, columns [cs + 2, cs + 62) and rows [j0, j0 + 20) of plane k.
 template <int NW, class IDX>
 __device__ __forceinline__ void hdiff_sift_tile(SiftTile& s, const double* __restrict__ inp,
                                                 const double* __restrict__ coeff, double* __restrict__ out, int ni, int nj,

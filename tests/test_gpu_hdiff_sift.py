@@ -36,7 +36,7 @@ def _check(inp, coeff, domain, halo, what, tune=SIFT):
 
 
 # one column, row and plane; a tile less, exactly and plus one; cut tiles in both directions
-@pytest.mark.parametrize("domain", [(1, 1, 1), (59, 15, 2), (60, 16, 2), (61, 17, 2), (121, 33, 3), (128, 128, 4), (7, 50, 2)])
+@pytest.mark.parametrize("domain", [(1, 1, 1), (59, 19, 2), (60, 20, 2), (61, 21, 2), (61, 17, 2), (121, 41, 3), (128, 128, 4), (7, 50, 2)])
 @pytest.mark.parametrize("halo", [(2, 2, 0), (3, 2, 1)])
 def test_tiles(domain, halo, lib):
     got, want, _ = _run_hdiff(domain, halo, tune=_native.tune(**SIFT), seed=sum(domain))

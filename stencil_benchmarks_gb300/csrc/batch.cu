@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(512, 1)
     const int first = tab->bucket_first[0], last = tab->bucket_first[kBuckets];
     const int64_t total = tab->bucket_items[0];
     if (total == 0) return;  // whole block, before any TMEM allocation
-    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    const int warp = uniform((int)(threadIdx.x >> 5)), lane = threadIdx.x & 31;
     const int nwarps = blockDim.x >> 5;
     const uint32_t tbase = tmem_alloc_all(reinterpret_cast<uint32_t*>(smem_tma), warp);
     const uint32_t tcol = tbase + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)((warp >> 2) * a.nt * kTmaBlockCols);
@@ -296,12 +296,15 @@ __global__ void __launch_bounds__(512, 1)
         const DevDomain& dm = tab->dom[lo];
         const int local = (int)((int64_t)item - dm.item_begin);
         const int i0 = v.live ? (local % dm.items_i) * 32 : 0, j = v.live ? local / dm.items_i : 0;
-        v.maps = dm.maps;
-#pragma unroll
-        for (int f = 0; f < kTmaFields; ++f) v.off[f] = dm.off[f];
+        const uintptr_t maps = (uintptr_t)dm.maps;
+        v.maps = (const CUtensorMap*)((uintptr_t)(uint32_t)uniform((int)(uint32_t)(maps >> 32)) << 32 |
+                                      (uint32_t)uniform((int)(uint32_t)maps));
         v.stage = (const S*)dm.f[0];
         v.out = (S*)dm.out;
         v.col0 = i0 + j * (int)dm.sj;
+#pragma unroll
+        for (int f = 0; f < kTmaFields; ++f) v.x[f] = uniform(v.col0 + dm.off[f]);
+        v.x[kTmaFields] = v.x[0] + uniform((int)dm.wsh);
         v.nvalid = min(32, dm.ni - i0);
         v.nk = dm.nk;
         v.sk = (int)dm.sk;

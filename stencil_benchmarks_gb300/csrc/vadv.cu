@@ -537,8 +537,8 @@ template <class S, int R, int NC>
 __global__ void __launch_bounds__(512, 1) vadv_tma_kernel(const __grid_constant__ TmaArgs<S, NC> a) {
     extern __shared__ __align__(128) unsigned char smem_tma[];
     using B = TmaBox<S, R>;
-    // warp-uniform by a broadcast, so that the tensor copies' operands can stay in uniform registers
-    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    // what the tensor copies' operands are computed from stays in uniform registers
+    const int warp = uniform((int)(threadIdx.x >> 5)), lane = threadIdx.x & 31;
     const int nwarps = blockDim.x >> 5;
     uint32_t* s_taddr = reinterpret_cast<uint32_t*>(smem_tma);
     const uint32_t tbase = tmem_alloc_all(s_taddr, warp);
@@ -554,11 +554,12 @@ __global__ void __launch_bounds__(512, 1) vadv_tma_kernel(const __grid_constant_
         v.live = group < ngroups;
         const int i0 = (group % gx) * 32, j = group / gx;
         v.maps = a.maps[c];
-#pragma unroll
-        for (int f = 0; f < kTmaFields; ++f) v.off[f] = a.off[c][f];
         v.stage = a.stage[c];
         v.out = a.out[c];
-        v.col0 = i0 + j * a.sj;
+        v.col0 = uniform(i0 + j * a.sj);
+#pragma unroll
+        for (int f = 0; f < kTmaFields; ++f) v.x[f] = v.col0 + a.off[c][f];
+        v.x[kTmaFields] = v.x[0] + a.wsh[c];
         v.nvalid = min(32, a.ni - i0);
         v.nk = a.nk;
         v.sk = a.sk;

@@ -74,11 +74,14 @@ struct TmaBox {
 };
 static_assert(TmaBox<float, 0>::W == 36 && TmaBox<bf16, 0>::W == 40 && TmaBox<bf16, -1>::W <= 256, "box widths");
 
+// a warp-uniform value, in a form that the compiler keeps in a uniform register
+__device__ __forceinline__ int uniform(int v) { return __reduce_max_sync(0xffffffffu, v); }
+
 // one solve of 32 columns: everything a warp needs to stage and compute it
 template <class S>
 struct TmaSolve {
     const CUtensorMap* maps;  // [kTmaFields]
-    int off[kTmaFields];      // element offset of each map's first level from its granule
+    int x[kTmaFields + 1];    // x of column col0 in each map, and of wcon's at the shift
     const S* stage;
     S* out;
     int col0, nvalid, nk, sk, wsh;
@@ -157,8 +160,8 @@ struct TmaPipe {
     __device__ __forceinline__ void init(unsigned char* m, unsigned char* bars, int lane_, uint32_t stages_, int stage_bytes,
                                          int polls_) {
         mem = m;
-        mem_s = (uint32_t)__cvta_generic_to_shared(m);
-        bar_s = (uint32_t)__cvta_generic_to_shared(bars);
+        mem_s = (uint32_t)uniform((int)__cvta_generic_to_shared(m));
+        bar_s = (uint32_t)uniform((int)__cvta_generic_to_shared(bars));
         stage_b = stage_bytes;
         lane = lane_;
         stages = stages_;
@@ -188,10 +191,9 @@ struct TmaPipe {
             expect(bar, (uint32_t)((far ? kTmaFields + 1 : kTmaFields) * (B::ROWB * kTmaLevels)));
 #pragma unroll
             for (int f = 0; f < kTmaFields; ++f)
-                tma_load_2d(v.maps + f, dst + (uint32_t)(f * B::BOXB), bar, box_x(v, v.off[f] + v.col0, blk),
-                            blk * kTmaLevels);
+                tma_load_2d(v.maps + f, dst + (uint32_t)(f * B::BOXB), bar, box_x(v, v.x[f], blk), blk * kTmaLevels);
             if (far)
-                tma_load_2d(v.maps, dst + (uint32_t)(kTmaFields * B::BOXB), bar, box_x(v, v.off[0] + v.col0 + v.wsh, blk),
+                tma_load_2d(v.maps, dst + (uint32_t)(kTmaFields * B::BOXB), bar, box_x(v, v.x[kTmaFields], blk),
                             blk * kTmaLevels);
         }
     }
@@ -202,7 +204,7 @@ struct TmaPipe {
         pfillr.next(kTmaPosStages);
         if (elect_one()) {
             expect(bar, (uint32_t)(B::ROWB * kTmaLevels));
-            tma_load_2d(v.maps + 2, dst, bar, box_x(v, v.off[2] + v.col0, blk), blk * kTmaLevels);
+            tma_load_2d(v.maps + 2, dst, bar, box_x(v, v.x[2], blk), blk * kTmaLevels);
         }
     }
     // Wait for the stage at position r of the ring whose first barrier is `bar`,
@@ -267,8 +269,8 @@ __device__ __forceinline__ bool vadv_tma_solve(TmaPipe<S, R>& pipe, const TmaSol
     const int drift = R < 0 ? v.drift : R;
     int el[kTmaFields + 1];
 #pragma unroll
-    for (int f = 0; f < kTmaFields; ++f) el[f] = f * B::BOXB + (((v.off[f] + v.col0) & (B::EPG - 1)) + lane) * B::ES;
-    el[kTmaFields] = v.wsh > 1 ? kTmaFields * B::BOXB + (((v.off[0] + v.col0 + v.wsh) & (B::EPG - 1)) + lane) * B::ES
+    for (int f = 0; f < kTmaFields; ++f) el[f] = f * B::BOXB + ((v.x[f] & (B::EPG - 1)) + lane) * B::ES;
+    el[kTmaFields] = v.wsh > 1 ? kTmaFields * B::BOXB + ((v.x[kTmaFields] & (B::EPG - 1)) + lane) * B::ES
                                : el[0] + v.wsh * B::ES;
     auto rd = [&](const unsigned char* st, int f, int q) -> float {  // field f at level q of the stage
         return cvt<float, S>(*reinterpret_cast<const S*>(st + el[f] + q * (B::ROWB + drift)));

@@ -17,6 +17,8 @@ constexpr int kBasicPK = 4;
 constexpr int kLapRows = 4;
 constexpr int kLapWarps = 4;
 constexpr int kLapPlanes = 2;
+// of eight points, those with one more float64 operation on the integer pipe
+constexpr int kLapMore = 3;
 // which Laplacian kernel runs when the tune names none
 constexpr int kLapDefaultVariant = SB_BASIC_MARCH;
 
@@ -87,13 +89,13 @@ __global__ void __launch_bounds__(256) basic_kernel(const S* __restrict__ inp, S
 // row is read once per strip plus the two rows beyond it; the i-neighbours are
 // loads of rows already fetched (L1 hits).  Same operations in the same order
 // as basic_point; PL places the float64 subtractions/additions (sites 0-7) on
-// the integer pipe.
-template <int MASK, class S, class C, int R, int PK, uint32_t PL>
+// the integer pipe for kLapMore of the eight points of 4 rows x 2 planes, PL2
+// for the others: the two pipes balance between whole numbers of operations.
+template <int MASK, class S, class C, int R, int PK, uint32_t PL, uint32_t PL2 = PL>
 __global__ void __launch_bounds__(256) lap_march_kernel(const S* __restrict__ inp, S* __restrict__ out, int ni,
                                                         int nj, int nk, int64_t si, int64_t sj, int64_t sk) {
     constexpr bool JN = (MASK & 2) != 0;
     using A = Ar<C>;
-    using X = Mix<C, PL>;
     constexpr int NR = JN ? R + 2 : R;  // rows held: j0-1 .. j0+R along j, else j0 .. j0+R-1
     constexpr int R0 = JN ? 1 : 0;      // index of row j0 in v[]
     const int i = blockIdx.x * 32 + threadIdx.x;
@@ -114,31 +116,36 @@ __global__ void __launch_bounds__(256) lap_march_kernel(const S* __restrict__ in
                           : C(0);
         }
     }
+    auto point = [&](auto mix, int r, int q) {
+        using X = decltype(mix);
+        const S* p = col + (int64_t)r * sj + (int64_t)q * sk;
+        const C two_x = A::template scale2<1>(v[q][r + R0]);
+        C acc = C(0);
+        bool first = true;
+        if (MASK & 1) {
+            const C t = X::sub(X::sub(two_x, ld<C, S>(p + si), site<0>{}), ld<C, S>(p - si), site<1>{});
+            acc = plus_zero<C>(t);
+            first = false;
+        }
+        if (MASK & 2) {
+            const C t = X::sub(X::sub(two_x, v[q][JN ? r + 2 : 0], site<2>{}), v[q][r], site<3>{});
+            acc = first ? plus_zero<C>(t) : X::add(acc, t, site<4>{});
+            first = false;
+        }
+        if (MASK & 4) {
+            const C t = X::sub(X::sub(two_x, ld<C, S>(p + sk), site<5>{}), ld<C, S>(p - sk), site<6>{});
+            acc = first ? plus_zero<C>(t) : X::add(acc, t, site<7>{});
+        }
+        st<S, C>(ocol + (int64_t)r * sj + (int64_t)q * sk, acc);
+    };
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         if (r < nrow) {
 #pragma unroll
             for (int q = 0; q < PK; ++q) {
                 if (kb + q < nk) {
-                    const S* p = col + (int64_t)r * sj + (int64_t)q * sk;
-                    const C two_x = A::template scale2<1>(v[q][r + R0]);
-                    C acc = C(0);
-                    bool first = true;
-                    if (MASK & 1) {
-                        const C t = X::sub(X::sub(two_x, ld<C, S>(p + si), site<0>{}), ld<C, S>(p - si), site<1>{});
-                        acc = plus_zero<C>(t);
-                        first = false;
-                    }
-                    if (MASK & 2) {
-                        const C t = X::sub(X::sub(two_x, v[q][r + 2], site<2>{}), v[q][r], site<3>{});
-                        acc = first ? plus_zero<C>(t) : X::add(acc, t, site<4>{});
-                        first = false;
-                    }
-                    if (MASK & 4) {
-                        const C t = X::sub(X::sub(two_x, ld<C, S>(p + sk), site<5>{}), ld<C, S>(p - sk), site<6>{});
-                        acc = first ? plus_zero<C>(t) : X::add(acc, t, site<7>{});
-                    }
-                    st<S, C>(ocol + (int64_t)r * sj + (int64_t)q * sk, acc);
+                    if ((r * PK + q) * kLapMore % 8 < kLapMore) point(Mix<C, PL>{}, r, q);  // known when unrolled
+                    else point(Mix<C, PL2>{}, r, q);
                 }
             }
         }
@@ -146,15 +153,19 @@ __global__ void __launch_bounds__(256) lap_march_kernel(const S* __restrict__ in
 }
 
 // float64 placements (sites of lap_march_kernel).  The default moves the second
-// subtraction of each axis to the integer pipe; presets of the along-x-and-y
+// subtraction of each axis to the integer pipe for three of eight points and
+// that of all axes but the first for the others; presets of the along-x-and-y
 // strips: 1 all fp64, 2 the closing addition, 3 the second subtraction of each
-// axis (the default), 4 those and the addition; other axis sets take the
-// default or, with a preset, run all fp64.  512x512x80 along x and y, five
-// operations per point: all on the fp64 pipe 247 us, one on the integer pipe
-// 207, two 187, three 262 (an fp64 operation takes about 41 us of that pipe, an
-// integer one 70 us of the ALU pipe); along one axis 103-108 against 126, along
-// three 297 against 366.
+// axis, 4 those and the addition; other axis sets take the default or, with a
+// preset, run all fp64.  An fp64 operation takes about 41 us of its pipe at
+// 512x512x80, an integer one 70 us of the ALU pipe.  Along x and y, of five
+// operations a point on the integer pipe: none 206 us, 1.13 163, 1.25 159, 1.38
+// 154, 1.5 154, 1.63 160, 1.75 167, 2 184 (ALU pipe 89%, fp64 56% busy); along
+// one axis 72-84 us (all fp64 87-90), along three 251 (326).
 constexpr uint32_t kLapDefaultSites = 0x4Au;
+constexpr uint32_t lap_fewer_sites(int mask) {
+    return kLapDefaultSites & ~(mask & 1 ? 0x02u : mask & 2 ? 0x08u : 0x40u);
+}
 constexpr uint32_t kLapPlacements[] = {0u, 0u, 0x10u, 0x0Au, 0x1Au};
 
 template <int MASK, class S, class C, int R, int PK>
@@ -168,7 +179,7 @@ int launch_lap_march_pl(int placement, const S* inp, S* out, int64_t ni, int64_t
         return SB_OK;
     };
     if constexpr (std::is_same<C, double>::value)
-        if (placement == 0) return go(lap_march_kernel<MASK, S, C, R, PK, kLapDefaultSites>);
+        if (placement == 0) return go(lap_march_kernel<MASK, S, C, R, PK, kLapDefaultSites, lap_fewer_sites(MASK)>);
     if constexpr (MASK == 3 && std::is_same<C, double>::value) {
         switch (placement) {
             case 2: return go(lap_march_kernel<MASK, S, C, R, PK, kLapPlacements[2]>);

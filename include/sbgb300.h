@@ -67,9 +67,11 @@ extern "C" {
 #define SB_VARIANT_AUTO 0  /* the library's choice, where the layout qualifies:
                             * hdiff: SIFT for float64, VSCAN for float32, bfloat16
                             * and float pairs, JSCAN otherwise (and for fixed64);
-                            * vadv: TMEM for float32 compute on >= 2048 column
-                            * groups (bfloat16: level stride a multiple of 8 bytes),
-                            * else SLAB / WSLAB when ccol/dcol are given, else SMEM */
+                            * vadv: TMEM staged by tensor copies for float32 compute
+                            * (i unit-stride, 9 <= nk <= 256, no shape in the tune;
+                            * shorter columns: TMEM with staged rows from 2048 column
+                            * groups on), else SLAB / WSLAB when ccol/dcol are given,
+                            * else SMEM                                              */
 #define SB_HDIFF_TILE 1   /* smem-staged k-plane tiles, lap/flx/fly once per point */
 #define SB_HDIFF_JSCAN 2  /* register j-march, i-neighbours by warp shuffles       */
 #define SB_HDIFF_TMA 3    /* TILE with inp k-planes staged by TMA (cp.async.bulk.tensor)
@@ -79,7 +81,9 @@ extern "C" {
                            * vector (block_x = strip width 32*V: 64 for 8-byte,
                            * 64 or 128 for 4-byte, 128 or 256 for 2-byte storage); i
                            * unit-stride, j/k strides multiples of the vector,
-                           * inp/coeff/out at one offset from a vector boundary */
+                           * inp/coeff/out at one offset from a vector boundary.
+                           * SB_VARIANT_AUTO also takes rows that no vectors fit (two
+                           * columns per lane, moved element by element)           */
 #define SB_HDIFF_SIFT 5   /* float64 storage and compute, any layout: fluxes that the
                            * limiter certainly zeroes are found in fixed point, the
                            * others and the points they feed computed in float64
@@ -99,11 +103,13 @@ extern "C" {
                            * in the tune picks WSLAB for 2/4-byte storage and SLAB
                            * for 8-byte storage when the layout qualifies and TMEM
                            * does not apply */
-#define SB_VADV_TMEM 5    /* float32 compute: WSLAB row staging, factors in tensor
-                           * memory (tcgen05.st / tcgen05.ld) instead of a slab; one
-                           * persistent block per SM; no scratch; needs i unit-stride
-                           * and 2 <= nk <= 256; unroll = ring depth 4, 8 or 16
-                           * (0: deepest that fits) */
+#define SB_VADV_TMEM 5    /* float32 compute: factors in tensor memory (tcgen05.st /
+                           * tcgen05.ld) instead of a slab; one persistent block per
+                           * SM; no scratch; needs i unit-stride and 2 <= nk <= 256.
+                           * Inputs staged by tensor copies, 8 levels at a time, for
+                           * nk >= 9; as rows (WSLAB's staging) for shorter columns or
+                           * when unroll names a ring depth (4, 8 or 16) or flags a
+                           * row-staging form                                      */
 
 /*
  * Launch tuning.  Zero in any field means "choose the default".  The
@@ -120,7 +126,7 @@ typedef struct sb_tune {
     int32_t k_per_cta; /* hdiff: k-planes per CTA                               */
     int32_t unroll;    /* STREAM: vectors per thread per iteration             */
     int32_t flags;     /* STREAM: bit0 streaming (evict-first) stores;
-                        * vadv TMEM: bit 10 / 11 stage through 32-bit shared
+                        * vadv TMEM: bit 10 / 11 stage rows through 32-bit shared
                         * addresses / generic pointers (neither: the default);
                         * float64 hdiff TMA / vadv SLAB / Laplacian strips:
                         * bits 4-7 pick which operations run as integer
@@ -265,8 +271,7 @@ int sb_vadv(int storage, int compute, const void* stage, const void* pos, const 
  * tensstage and out are arrays of three pointers (u, v, w), every field with
  * the same layout; u reads wcon at (i+1, j), v at (i, j+1), w at (i, j).
  * With float32 compute on a layout the tensor-memory form takes (variant
- * AUTO with no explicit shape and at least 2048 column groups of 32, or
- * SB_VADV_TMEM) one launch solves the three components of each column group
+ * AUTO with no explicit shape, or SB_VADV_TMEM) one launch solves the three components of each column group
  * in turn, so wcon comes from HBM once; otherwise one sb_vadv launch per
  * component.  Same bits either way. */
 int sb_vadv3(int storage, int compute, const void* const* stage, const void* const* pos,
@@ -280,7 +285,8 @@ int sb_vadv3(int storage, int compute, const void* const* stage, const void* con
  * same hdiff / vadv computations.  A batch holds up to max_domains domains of
  * one (storage, compute) form; sb_batch_launch runs all of them in one graph
  * launch (captured on the first launch) of persistent kernels -- one for the
- * hdiff domains, one per nk bucket for the vadv domains, running side by side
+ * hdiff domains, one for the vadv domains (float32 compute, i unit-stride, at
+ * least 17 levels each) or one per nk bucket of them, running side by side
  * -- that pull work items from device-side queues.  Results
  * are bit-identical to sb_hdiff / sb_vadv on the same domain.  The domain
  * table lives in pinned host memory and is copied by each launch: do not

@@ -2,8 +2,8 @@
 
 ``Batch`` wraps ``sb_batch_*``: a fixed-capacity domain table, device-side
 work queues and a CUDA graph (table upload -> queue reset -> persistent hdiff
-kernel side by side with one persistent vadv kernel per nk bucket) that
-``launch()`` replays.  Every domain
+kernel side by side with one persistent vadv kernel, or one per nk bucket)
+that ``launch()`` replays.  Every domain
 of a batch has the same storage/compute form.  Results are bit-identical to
 launching ``kernels.hdiff`` / ``kernels.vadv`` on each domain.
 

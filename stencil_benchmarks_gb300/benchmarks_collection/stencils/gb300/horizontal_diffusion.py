@@ -9,8 +9,9 @@ algorithm).  Every class derives from the reference's
 * ``JScan``      -- warp j-march with shuffles (HBM-efficient float32 form);
 * ``Tile``       -- shared-memory k-plane tiles (fewest fp64 operations);
 * ``TmaTile``    -- the tiles with each k-plane brought in by the tensor
-  memory accelerator, double-buffered (fastest exact float64 form; needs
-  j/k strides that are multiples of 16 bytes, hence alignment 64 by default);
+  memory accelerator, double-buffered (needs j/k strides that are multiples
+  of 16 bytes, hence alignment 64 by default; the library's own choice for
+  float64 evaluates only what the limiter lets through and is faster);
 * ``VectorScan`` -- the j-march with several columns per lane moved as one
   aligned vector (fastest bfloat16-storage and float-pair form).
 """

@@ -20,8 +20,8 @@ cuda_hip/templates/vertical_advection_localmemmerged.j2).
 * ``NoAlloc``       -- factors in the library's static scratch array
   (``sb_vadv_noalloc``), for callers that cannot allocate device memory;
 * ``TensorMem``     -- float32 compute: rows staged per warp, factors in the
-  SM's tensor memory (one persistent block per SM; fastest float32 and, with
-  16-byte-multiple level strides, bfloat16 form).
+  SM's tensor memory (one persistent block per SM; the library's own choice
+  for float32 compute stages by tensor copies instead and is faster).
 """
 
 from __future__ import annotations
@@ -118,7 +118,7 @@ class GlobalScratch(VerticalAdvectionMixin, base.VerticalAdvectionStencil):
 
 class Slab(VerticalAdvectionMixin, base.VerticalAdvectionStencil):
     block_size = Parameter("threads per block along i (32 or 64), persistent blocks per SM (0: the library's "
-                           "choice: 24 when the float64 products run in integer arithmetic, otherwise as many as "
+                           "choice: 28 when the float64 products run in integer arithmetic, otherwise as many as "
                            "keep the factor slabs within half of L2)", (32, 0))
     unroll_factor = Parameter("levels of inputs kept in flight (1 with 32-thread blocks, 2, 4 or 8)", 1,
                               choices=[1, 2, 4, 8])
@@ -175,7 +175,8 @@ class TensorMem(VerticalAdvectionMixin, base.VerticalAdvectionStencil):
         return _native.tune(variant=_native.VADV_TMEM, unroll=self.unroll_factor)
 
     def tune_candidates(self):
-        return [_native.tune(variant=_native.VADV_TMEM, unroll=u) for u in (4, 8, 16)]
+        # 0: staged by tensor copies instead of rows
+        return [_native.tune(variant=_native.VADV_TMEM, unroll=u) for u in (0, 4, 8, 16)]
 
     def launch_component(self, f, named, shift, timed):
         return kernels.vadv(*f, named["wcon"], shift, compute=self.compute, tune=self.current_tune(), timed=timed)

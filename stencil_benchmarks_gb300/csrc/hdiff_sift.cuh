@@ -34,8 +34,8 @@
 // quarter) are computed in full (hdiff_dense_tile).
 //
 // 512x512x80, U[0, 1): 189 us against 547 for the TMA tile, which computes
-// everything; 3.1 fp64 instructions per point instead of 11.6, that pipe 54% and
-// the issue slots 58% busy.  128x128x64: 18.9 us against 36.7.  On other fields,
+// everything; 3.1 fp64 instructions per point instead of 11.6, that pipe 56% and
+// the issue slots 71% busy.  128x128x64: 18.5 us against 36.7.  On other fields,
 // 512x512x40, against the tile's 278 us: 105 on U[0, 1) and U[-1, 1), 91 on a
 // smooth field, 124 to 227 on a ramp or a smooth field with noise, 293 where
 // half the fluxes pass and every tile is computed in full after all.

@@ -17,7 +17,7 @@
 // mod 16 bytes further right than level k - 1: the boxes are 7 * drift bytes
 // wider, a stage's box starts 8 * drift bytes (a multiple of 16) further right
 // than the one before, and row q of a box begins q * drift bytes into it.
-// (512x512x80 bfloat16 with drift 8: 77 us; with two maps of every other level
+// (512x512x80 bfloat16 with drift 8 at 11 warps: 77 us; with two maps of every other level
 // instead, twice the copies, 91 us.)
 //
 // Stages form a ring per warp that runs on across solves: a freed stage is
@@ -26,13 +26,16 @@
 // backward sweep.  pos returns for the backward sweep through a second ring.
 // The factors of a warp's first nt level blocks live in TMEM, those of the
 // others in shared memory: TMEM alone would hold 12 warps per SM at 80 levels
-// and 4 from 129 levels on.
+// and 4 from 137 levels on.  The last block's stay in registers, as the backward
+// sweep starts with them; the 2 KB a warp that this frees let 14 warps of two
+// stages share an SM at 80 levels (8192 column groups in 4 rounds instead of 5:
+// bfloat16 76 -> 72 us, float32 100 either way).
 // All waits are bounded (see TmaPipe::wait).
 // Bound, 512x512x80: float32 HBM (5.0 TB/s of compulsory bytes, 75% of the
 // measured copy rate; fewer warps or deeper rings change it by 2%), bfloat16 the
-// issue slots and the recurrence's latency at 11 warps per SM.  Against the
+// issue slots and the recurrence's latency at 14 warps per SM.  Against the
 // cp.async form: float32 131 -> 100 us (odd planes 153 -> 110), bfloat16
-// 113 -> 77 (odd planes 151 -> 84; aligned rows 85 -> 40 at 510x254x80),
+// 113 -> 72 (odd planes 151 -> 84; aligned rows 85 -> 40 at 510x254x80),
 // 400x300x137 170 -> 99 and 189 -> 89, u, v, w of 256x256x80 fused 144 -> 83.
 #pragma once
 
@@ -254,8 +257,8 @@ __device__ __forceinline__ float rcp_in_range(float d) {
 // Solve `v` (its first `stages` level blocks are in the ring or on their
 // way); `next` is the warp's next solve, `FillNext(blk)` fills its block.
 // stage0: stage(k = 0) of this lane's column, on return that of `next`.
-// Factors of block b: TMEM columns tcol + 16 * b for b < nt, else shared memory
-// fmem + (b - nt) * 2 KB.  Returns false when a wait gave up: nothing is in the
+// Factors of block b: registers for the last block, TMEM columns tcol + 16 * b
+// for b < nt, else shared memory fmem + (b - nt) * 2 KB.  Returns false when a wait gave up: nothing is in the
 // rings then.
 template <class S, int R, class FillNext>
 __device__ __forceinline__ bool vadv_tma_solve(TmaPipe<S, R>& pipe, const TmaSolve<S>& v, const TmaSolve<S>& next,
@@ -362,7 +365,9 @@ __device__ __forceinline__ bool vadv_tma_solve(TmaPipe<S, R>& pipe, const TmaSol
                 }
             }
         }
-        if (b < nt) {
+        if (b == nblk - 1) {
+            // the backward sweep starts with them
+        } else if (b < nt) {
             tmem_st16(tcol + (uint32_t)(kTmaBlockCols * b), fac);
         } else {
 #pragma unroll
@@ -385,6 +390,8 @@ __device__ __forceinline__ bool vadv_tma_solve(TmaPipe<S, R>& pipe, const TmaSol
     float data = dp;
     if (valid) st<S, float>(out + (nk - 1) * v.sk, A::mul(dtr, A::sub(data, plast)));
     uint32_t fr[2 * L];
+#pragma unroll
+    for (int q = 0; q < 2 * L; ++q) fr[q] = __float_as_uint(fac[q]);
     auto factors = [&](int b) {  // on their way into fr
         if (b < nt) {
             tmem_ld16_issue(tcol + (uint32_t)(kTmaBlockCols * b), fr);
@@ -393,7 +400,6 @@ __device__ __forceinline__ bool vadv_tma_solve(TmaPipe<S, R>& pipe, const TmaSol
             for (int q = 0; q < 2 * L; ++q) fr[q] = __float_as_uint(fmem[((b - nt) * 2 * L + q) * 32 + lane]);
         }
     };
-    factors(nblk - 1);
     for (int b = nblk - 1; b >= 0; --b) {
         if (!pipe.ready_pos()) {
             pipe.abandon(status, next.live ? (int)pipe.stages : 0, min(kTmaPosStages, b + 1));
@@ -472,8 +478,8 @@ inline TmaShape tma_shape(bool far, int64_t nk, int64_t ngroups, int sms, int sm
     for (int stages = kTmaMaxStages; stages >= 2; --stages) {
         if (nk < tma_min_levels(stages)) continue;
         for (int quarter = 1; quarter <= 4; ++quarter) {  // warps that share a lane quarter of TMEM
-            const int nt = std::min(nblk, 512 / kTmaBlockCols / quarter);
-            const int bytes = B::rings_bytes(far, stages) + (nblk - nt) * kTmaBlockBytes;
+            const int nt = std::min(nblk - 1, 512 / kTmaBlockCols / quarter);  // the last block's stay in registers
+            const int bytes = B::rings_bytes(far, stages) + (nblk - 1 - nt) * kTmaBlockBytes;
             const int64_t fit = std::min<int64_t>(4 * quarter, (smem_optin - 16 - 128) / (bytes + B::BAR_BYTES));
             if (fit < 1) continue;
             const int64_t rounds = ceil_div(ngroups, sms * fit);

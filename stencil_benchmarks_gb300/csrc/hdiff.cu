@@ -581,6 +581,9 @@ int launch_typed(const void* inp, const void* coeff, void* out, int64_t ni, int6
     // columns per lane, packed float32 arithmetic) issue fewer instructions per
     // point than JSCAN (44 vs 62 us, 273 vs 313 us and, with V = 2, 46 vs 53 us at
     // 512x512x80; 56 and 49 with scalar arithmetic and rows loaded U at a time).
+    // float32 loads 8 rows at a time: 43.3 us at 512x512x80, 4 rows 46.0, 2 49.4,
+    // 1 59.7 (79 and 84 us with 8 and 4 at 1024x1024x40, the same at 128x128x64);
+    // the 64 registers are what that costs.  16-row tiles: 8 rows 45.4, 32 45.4.
     if constexpr (std::is_same<S, bf16>::value || std::is_same<C, f32x2>::value) {
         if (variant == SB_VARIANT_AUTO) {
             constexpr int V = sizeof(S) == 8 ? 2 : 4;
@@ -590,7 +593,7 @@ int launch_typed(const void* inp, const void* coeff, void* out, int64_t ni, int6
     }
     if constexpr (std::is_same<S, float>::value && std::is_same<C, float>::value) {
         if (variant == SB_VARIANT_AUTO) {
-            const int rc_v = launch_vscan<S, C, 2, true>(inp, coeff, out, ni, nj, nk, si, sj, sk, 2, 16, 1, 4, stream, p);
+            const int rc_v = launch_vscan<S, C, 2, true>(inp, coeff, out, ni, nj, nk, si, sj, sk, 2, 16, 1, 8, stream, p);
             if (rc_v != SB_ERR_UNSUPPORTED) return rc_v;
         }
     }

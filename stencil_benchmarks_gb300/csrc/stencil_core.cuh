@@ -224,8 +224,8 @@ __device__ __forceinline__ void hdiff_vscan_strip(const S* __restrict__ inp, con
     // Rows j + 2 of inp and j of coeff of U output rows.  Two-byte storage: always
     // the next U rows in flight, each reloaded when used (512x512x80 bfloat16
     // 44 us, 49 loading U at a time).  Wider storage: U rows loaded together, then
-    // computed (float32 48 us, 52 with the rows always in flight, whose separate
-    // waits outnumber the hardware's scoreboards).
+    // computed (float32, U = 4: 46 us, 52 with the rows always in flight, whose
+    // separate waits outnumber the hardware's scoreboards).
     constexpr bool RING = sizeof(S) == 2;
     Row rin[U], rcf[U];
     auto load_rows = [&](int j) {  // of output rows j .. j + U - 1

@@ -246,7 +246,9 @@ int sb_average(int storage, int compute, const void* inp, void* out, int64_t ni,
                const sb_tune* tune, void* stream, double* time_s);
 
 /* ---- horizontal diffusion (reference: stencils/cuda_hip/horizontal_diffusion.py,
- *      oracle stencils/base.py:276-311).  Needs a halo of >= 2 in i and j.    */
+ *      oracle stencils/base.py:276-311).  Needs a halo of >= 2 in i and j.
+ *      out may be coeff itself (any other overlap is not allowed), here and in
+ *      a batch.                                                                */
 int sb_hdiff(int storage, int compute, const void* inp, const void* coeff, void* out,
              int64_t ni, int64_t nj, int64_t nk, int64_t si, int64_t sj, int64_t sk,
              const sb_tune* tune, void* stream, double* time_s);

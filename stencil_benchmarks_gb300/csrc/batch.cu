@@ -155,9 +155,13 @@ __global__ void __launch_bounds__(32 * kSiftWarps, 9)
         const int k1 = min(dm.nk, k0 + planes);
         for (int k = k0; k < k1; ++k) {
             if (k > k0) __syncthreads();
-            hdiff_sift_tile<kSiftWarps, IDX>(tile, (const double*)dm.f[0], (const double*)dm.f[1], (double*)dm.out, dm.ni,
-                                             dm.nj, (IDX)dm.si, (IDX)dm.sj, (IDX)dm.sk, strip * kSiftOut - 2,
-                                             jb * kSiftRows, k, threadIdx.x >> 5, threadIdx.x & 31);
+            const int cs = strip * kSiftOut - 2, j0 = jb * kSiftRows, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+            if (dm.f[1] == dm.out)
+                hdiff_in_place_tile<kSiftWarps, IDX>(tile, (const double*)dm.f[0], (double*)dm.out, dm.ni, dm.nj, (IDX)dm.si,
+                                                     (IDX)dm.sj, (IDX)dm.sk, cs, j0, k, warp, lane);
+            else
+                hdiff_sift_tile<kSiftWarps, IDX>(tile, (const double*)dm.f[0], (const double*)dm.f[1], (double*)dm.out, dm.ni,
+                                                 dm.nj, (IDX)dm.si, (IDX)dm.sj, (IDX)dm.sk, cs, j0, k, warp, lane);
         }
     }
 }

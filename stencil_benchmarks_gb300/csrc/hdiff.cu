@@ -235,13 +235,18 @@ int launch_vscan(const void* inp, const void* coeff, void* out, int64_t ni, int6
 }
 
 // SIFT: one block per tile of 60 x 20 outputs of one plane (hdiff_sift.cuh).
-template <class IDX>
+// IN_PLACE: out is coeff.
+template <class IDX, bool IN_PLACE>
 __global__ void __launch_bounds__(32 * kSiftWarps, 9)
     hdiff_sift_kernel(const double* __restrict__ inp, const double* __restrict__ coeff, double* __restrict__ out, int ni,
                       int nj, IDX si, IDX sj, IDX sk) {
     __shared__ __align__(16) SiftTile tile;
-    hdiff_sift_tile<kSiftWarps, IDX>(tile, inp, coeff, out, ni, nj, si, sj, sk, (int)blockIdx.x * kSiftOut - 2,
-                                     (int)blockIdx.y * kSiftRows, (int)blockIdx.z, threadIdx.x >> 5, threadIdx.x & 31);
+    const int cs = (int)blockIdx.x * kSiftOut - 2, j0 = (int)blockIdx.y * kSiftRows, k = (int)blockIdx.z;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if constexpr (IN_PLACE)
+        hdiff_in_place_tile<kSiftWarps, IDX>(tile, inp, out, ni, nj, si, sj, sk, cs, j0, k, warp, lane);
+    else
+        hdiff_sift_tile<kSiftWarps, IDX>(tile, inp, coeff, out, ni, nj, si, sj, sk, cs, j0, k, warp, lane);
 }
 
 int launch_sift(const void* inp, const void* coeff, void* out, int64_t ni, int64_t nj, int64_t nk, int64_t si, int64_t sj,
@@ -250,12 +255,14 @@ int launch_sift(const void* inp, const void* coeff, void* out, int64_t ni, int64
     if (gy > p->max_grid_y || nk > p->max_grid_z) return SB_ERR_UNSUPPORTED;
     const dim3 grid((unsigned)gx, (unsigned)gy, (unsigned)nk), block(32 * kSiftWarps);
     const int64_t reach = (ni + 2 + kSiftCols) * std::abs(si) + (nj + 2 + kSiftRows) * std::abs(sj) + nk * std::abs(sk);
-    if (reach < (1LL << 31))
-        hdiff_sift_kernel<int><<<grid, block, 0, stream>>>((const double*)inp, (const double*)coeff, (double*)out, (int)ni,
-                                                           (int)nj, (int)si, (int)sj, (int)sk);
-    else
-        hdiff_sift_kernel<int64_t><<<grid, block, 0, stream>>>((const double*)inp, (const double*)coeff, (double*)out,
-                                                               (int)ni, (int)nj, si, sj, sk);
+    auto go = [&](auto kernel, auto idx) {
+        using IDX = decltype(idx);
+        kernel<<<grid, block, 0, stream>>>((const double*)inp, (const double*)coeff, (double*)out, (int)ni, (int)nj, (IDX)si,
+                                           (IDX)sj, (IDX)sk);
+    };
+    const bool in_place = out == coeff;
+    if (reach < (1LL << 31)) go(in_place ? hdiff_sift_kernel<int, true> : hdiff_sift_kernel<int, false>, int());
+    else go(in_place ? hdiff_sift_kernel<int64_t, true> : hdiff_sift_kernel<int64_t, false>, int64_t());
     return SB_OK;
 }
 
@@ -556,8 +563,9 @@ int launch_typed(const void* inp, const void* coeff, void* out, int64_t ni, int6
     // in hdiff_sift.cuh).  Otherwise TILE computes every lap/flx/fly once per
     // tile (fewest fp64 operations); fp32 and float-pair compute are
     // bound by instruction issue: JSCAN (shuffles, no block barriers) is faster.
-    // With a placement preset of its sites asked for, or a domain too large for
-    // SIFT's grid, the TMA-staged tile is the fastest that computes everything (its
+    // With a placement preset of its sites asked for, a domain too large for
+    // SIFT's grid, or out the same field as coeff (where SIFT computes every tile
+    // in full), the TMA-staged tile is the fastest that computes everything (its
     // loads leave the issue slots to the fp64 arithmetic and overlap the
     // previous plane's compute); it needs TMA-describable strides, else TILE.
     // 128 x 4 threads, 16-row tiles, one k-plane per block at 512x512x80:
@@ -565,7 +573,7 @@ int launch_typed(const void* inp, const void* coeff, void* out, int64_t ni, int6
     // 24 and 32 rows 652-716 (two blocks per SM no longer fit).
     const bool auto_tile = variant == SB_VARIANT_AUTO && std::is_same<C, double>::value;
     if constexpr (std::is_same<S, double>::value && std::is_same<C, double>::value) {
-        if (variant == SB_HDIFF_SIFT || (variant == SB_VARIANT_AUTO && placement == 0)) {
+        if (variant == SB_HDIFF_SIFT || (variant == SB_VARIANT_AUTO && placement == 0 && out != coeff)) {
             const int rc_sift = launch_sift(inp, coeff, out, ni, nj, nk, si, sj, sk, stream, p);
             SB_CHECK(rc_sift != SB_ERR_UNSUPPORTED || variant == SB_VARIANT_AUTO, SB_ERR_UNSUPPORTED,
                      "hdiff SIFT: domain too large for its launch grid");

@@ -31,7 +31,10 @@
 // finite or x is -0.
 // Tiles with an inf or nan, a value of 2^1017 or more, all values below 2^-474,
 // a -0, a coefficient that is not finite, or more than kSiftCap open fluxes (a
-// quarter) are computed in full (hdiff_dense_tile).
+// quarter) are computed in full (hdiff_dense_tile).  So is every tile where out
+// is coeff itself (hdiff_in_place_tile): step 1 would overwrite the coefficients
+// that step 4 reads; computed in full, each is read by the lane that then writes
+// its point.
 //
 // 512x512x80, U[0, 1): 189 us against 547 for the TMA tile, which computes
 // everything; 3.1 fp64 instructions per point instead of 11.6, that pipe 56% and
@@ -137,7 +140,34 @@ __device__ __noinline__ void hdiff_dense_tile(const double* tile, const double* 
     }
 }
 
-// The NW warps of a block, columns [cs + 2, cs + 62) and rows [j0, j0 + 20) of plane k.
+// the tile at smem computed in full, each of the NW warps a piece of its rows
+template <int NW, class IDX>
+__device__ __forceinline__ void hdiff_dense_pieces(const double* tile, const double* __restrict__ coeff,
+                                                   double* __restrict__ out, int ni, int cs, IDX si, IDX sj, IDX base, int warp,
+                                                   int lane, int nrow) {
+    const int piece = (nrow + NW - 1) / NW, q0 = warp * piece, n = min(piece, nrow - q0);
+    if (n > 0) hdiff_dense_tile<IDX>(tile + q0 * kSiftCols, coeff, out, ni, cs, si, sj, base + (IDX)q0 * sj, lane, n);
+}
+
+// A tile of hdiff_sift_tile's shape where out is coeff.  A function of its own: a
+// run-time condition on the store in hdiff_sift_tile's first step made every call
+// slower (512x512x80: 254 us instead of 189).
+template <int NW, class IDX>
+__device__ __noinline__ void hdiff_in_place_tile(SiftTile& s, const double* __restrict__ inp, double* out, int ni, int nj,
+                                                 IDX si, IDX sj, IDX sk, int cs, int j0, int k, int warp, int lane) {
+    const int nrow = min(kSiftRows, nj - j0);
+    const IDX base = (IDX)k * sk + (IDX)cs * si + (IDX)j0 * sj;
+    for (int t = warp; t < nrow + 4; t += NW)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int c = lane + 32 * h;
+            s.x[t * kSiftCols + c] = cs + c <= ni + 1 ? __ldg(inp + (base + (IDX)c * si + (IDX)(t - 2) * sj)) : 0.0;
+        }
+    __syncthreads();
+    hdiff_dense_pieces<NW, IDX>(s.x, out, out, ni, cs, si, sj, base, warp, lane, nrow);
+}
+
+// The NW warps of a block, columns [cs + 2, cs + 62) and rows [j0, j0 + 20) of plane k; out is not coeff.
 template <int NW, class IDX>
 __device__ __forceinline__ void hdiff_sift_tile(SiftTile& s, const double* __restrict__ inp,
                                                 const double* __restrict__ coeff, double* __restrict__ out, int ni, int nj,
@@ -242,8 +272,7 @@ __device__ __forceinline__ void hdiff_sift_tile(SiftTile& s, const double* __res
     }
     const int total = __shfl_sync(0xffffffffu, sum, 31);
     if (!plain || total > kSiftCap) {
-        const int piece = (nrow + NW - 1) / NW, q0 = warp * piece, n = min(piece, nrow - q0);
-        if (n > 0) hdiff_dense_tile<IDX>(s.x + q0 * W, coeff, out, ni, cs, si, sj, base + (IDX)q0 * sj, lane, n);
+        hdiff_dense_pieces<NW, IDX>(s.x, coeff, out, ni, cs, si, sj, base, warp, lane, nrow);
         return;
     }
     if (total == 0) return;

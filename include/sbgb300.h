@@ -152,16 +152,19 @@ int sb_synchronize(void);
  * (alone and in batches), which wait on an mbarrier for each plane or block of
  * levels.  A wait gives up after a bounded number of polls; the whole thread
  * block (vadv: the warp) then stops before storing what it waited for, waits
- * (bounded) for the copies it still has in flight and sets a process-wide
- * status word held in page-locked, device-mapped host memory (allocated by the
- * first such launch: make the first sb_hdiff call before any stream capture;
- * sb_vadv takes a form without waits when its first call is captured).  The
- * give-up is reported as SB_ERR_TIMEOUT, and the word cleared, by the first of:
- * a timed sb_hdiff, sb_vadv, sb_vadv3 or sb_batch_launch call (after its
- * launch), the next such call (before it launches anything), sb_synchronize,
- * sb_stream_synchronize,
- * sb_event_synchronize, or sb_kernel_status.  No reference counterpart (its
- * kernels do not wait on the device).
+ * (bounded) for the copies it still has in flight and sets a status word in
+ * page-locked, device-mapped host memory (allocated by the first such launch:
+ * make the first TMA sb_hdiff call before any stream capture; sb_vadv takes a
+ * form without waits when its first call is captured).  Each stream and each
+ * batch has its own word.  The give-up is reported as SB_ERR_TIMEOUT, and the
+ * word cleared, by the first of: a timed sb_hdiff, sb_vadv, sb_vadv3 or
+ * sb_batch_launch call (after its launch), the next such call on the same
+ * stream or of the same batch (before it launches anything; calls on other
+ * streams are not affected), sb_synchronize, sb_stream_synchronize,
+ * sb_event_synchronize (each reports any stream's), or sb_kernel_status.  A
+ * launch captured into the caller's own graph counts as one of the stream it
+ * was captured from.  No reference counterpart (its kernels do not wait on the
+ * device).
  * sb_kernel_status: SB_ERR_TIMEOUT if a launch has given up since the last
  * report, else SB_OK; does not synchronise.
  * sb_debug_wait_limit: testing aid, the polls of each first wait (0: give up

@@ -517,7 +517,7 @@ struct sb_batch {
     // (drift class + kTmaClasses where a domain reads wcon at j + 1; -1: not this form)
     int use_tma = -1, graph_tma = -1;
     TmaShape tma_shapes[2 * kTmaClasses] = {};
-    int* status = nullptr;
+    BatchStatus status;  // its word lies behind host_table
     int graph_polls = 0;
 };
 
@@ -534,7 +534,8 @@ void release(sb_batch* b) {
         if (e) cudaEventDestroy(e);
     if (b->counters) cudaFree(b->counters);
     if (b->slab_mem) cudaFree(b->slab_mem);
-    if (b->dev_table) cudaFree(b->dev_table);
+    if (b->dev_table) cudaFree(b->dev_table);  // (after which no launch of the batch runs any more)
+    if (b->status.word) unlist_batch_status(&b->status);
     if (b->host_table) cudaFreeHost(b->host_table);
     delete b;
 }
@@ -600,7 +601,7 @@ int capture_graph(sb_batch* b) {
     if (b->use_tma >= 0) {
         const TmaClass& c = k.tma[b->use_tma % kTmaClasses];
         const TmaShape& sh = b->tma_shapes[b->use_tma];
-        ta = {sh.nt, sh.stages, c.stage_bytes(b->use_tma >= kTmaClasses), sh.warp_bytes, wait_polls(), b->status};
+        ta = {sh.nt, sh.stages, c.stage_bytes(b->use_tma >= kTmaClasses), sh.warp_bytes, wait_polls(), b->status.word};
         tma_smem = std::max<size_t>(c.ring_offset(sh.warps) + (size_t)sh.warps * sh.warp_bytes, 120 * 1024);
         SB_CUDA(cudaFuncSetAttribute(c.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tma_smem));
         b->graph_polls = ta.polls;
@@ -740,11 +741,6 @@ int sb_batch_create(sb_batch** out, int storage, int compute, int max_domains, i
         for (int q = 0; q < 2 * kTmaClasses; ++q)
             if (k.tma[q % kTmaClasses].run && max_nk >= tma_min_levels(2))
                 b->tma_shapes[q] = k.tma[q % kTmaClasses].shape(q >= kTmaClasses, max_nk, p->sm_count, p->smem_optin);
-        rc = status_word(&b->status);
-        if (rc) {
-            release(b);
-            return rc;
-        }
     }
     size_t slab_total = 0;
     size_t slab_off[kBuckets] = {};
@@ -754,7 +750,8 @@ int sb_batch_create(sb_batch** out, int storage, int compute, int max_domains, i
             slab_total += (2 * (size_t)b->cap[q] * b->vadv_grid[q] * b->vadv_block * k.compute_bytes + 255) / 256 * 256;
         }
     }
-    cudaError_t e = cudaMallocHost((void**)&b->host_table, table_bytes(max_domains));
+    const size_t status_at = ceil_div((int64_t)table_bytes(max_domains), (int64_t)128) * 128;  // a cache line of its own
+    cudaError_t e = cudaMallocHost((void**)&b->host_table, status_at + 128);
     if (e == cudaSuccess) e = cudaMalloc((void**)&b->dev_table, table_bytes(max_domains));
     if (e == cudaSuccess) e = cudaMalloc((void**)&b->counters, sizeof(unsigned long long) * (1 + kBuckets));
     if (e == cudaSuccess && slab_total) {
@@ -775,7 +772,9 @@ int sb_batch_create(sb_batch** out, int storage, int compute, int max_domains, i
         return fail(e == cudaErrorMemoryAllocation ? SB_ERR_NOMEM : SB_ERR_CUDA, "batch allocation failed: %s",
                     cudaGetErrorString(e));
     }
-    memset(b->host_table, 0, table_bytes(max_domains));
+    memset(b->host_table, 0, status_at + 128);
+    b->status.word = (int*)((char*)b->host_table + status_at);
+    list_batch_status(&b->status);
     b->host_table->rows = b->tune.hdiff_rows;
     b->host_table->planes = b->tune.hdiff_planes;
     *out = b;
@@ -933,8 +932,8 @@ int sb_batch_launch(sb_batch* b, void* stream, double* time_s) {
     SB_CUDA(cudaGetDevice(&dev));
     SB_CHECK(dev == b->device, SB_ERR_INVALID, "batch was created on device %d, current device is %d", b->device,
              dev);
-    // a give-up of an earlier launch is reported before anything new runs
-    int rc = take_wait_status();
+    // a give-up of an earlier launch of the batch or on the stream is reported before anything new runs
+    int rc = begin_batch_launch(&b->status, (cudaStream_t)stream);
     if (rc) return rc;
     if (!b->exec || b->graph_idx64 != b->idx64 || b->graph_tmem != b->use_tmem || b->graph_tma != b->use_tma ||
         (b->use_tma >= 0 && b->graph_polls != wait_polls())) {
@@ -945,7 +944,7 @@ int sb_batch_launch(sb_batch* b, void* stream, double* time_s) {
         SB_CUDA(cudaGraphLaunch(b->exec, (cudaStream_t)stream));
         return SB_OK;
     });
-    if (rc == SB_OK && time_s && b->use_tma >= 0) rc = take_wait_status();
+    if (rc == SB_OK && time_s && b->use_tma >= 0) rc = take_stream_status((cudaStream_t)stream);
     return rc;
 }
 

@@ -53,15 +53,41 @@ int device_props(const DeviceProps** out);
 // ---------------------------------------------------------------------------
 // bounded device-side waits
 // ---------------------------------------------------------------------------
-// A kernel whose wait gives up sets a process-wide status word that lives in
-// page-locked, device-mapped host memory (allocated on the first call of
-// status_word), so the host reads it without synchronising.  take_wait_status
-// returns SB_ERR_TIMEOUT (with a message) and clears the word if it was set.
-int status_word(int** device_ptr);
-int take_wait_status();
+// A kernel whose wait gives up sets a status word that lives in page-locked,
+// device-mapped host memory, so the host reads it without synchronising.  Each
+// stream has a word of its own for its plain launches and each batch one for
+// its own, so that a call is refused for an earlier launch on its own stream
+// only.  Launches captured into a graph count as ones of the stream they were
+// captured from; the default streams of all devices share a word, and so do
+// streams beyond the table.
+//
+// status_word: the word for a launch on `stream`.
+// take_stream_status: SB_ERR_TIMEOUT (with a message), and the words cleared,
+// if a launch on `stream` (a batch's last one among them) has given up.
+// take_status: the same for all words but those of private streams.
+int status_word(cudaStream_t stream, int** device_ptr);
+int take_stream_status(cudaStream_t stream);
+int take_status();
 // Whether status_word can be called for a launch on `stream`: its first call
 // allocates, which a stream under capture does not allow.
 bool status_ready(cudaStream_t stream);
+// A private stream's give-ups are reported by take_stream_status only: for an
+// owner that has to hear of each one itself.
+int make_stream_private(cudaStream_t stream);
+// Before a stream is destroyed: its word may serve another one.
+void forget_stream(cudaStream_t stream);
+// A batch's word and the stream of its last launch, listed while the batch
+// lives (a give-up not reported by its end goes to the shared word).
+struct BatchStatus {
+    int* word = nullptr;
+    cudaStream_t stream = nullptr;
+    bool launched = false;
+    BatchStatus *next = nullptr, *prev = nullptr;
+};
+void list_batch_status(BatchStatus* b);
+void unlist_batch_status(BatchStatus* b);
+// before a launch: reports what the batch's earlier ones or the stream's have left, else notes the stream
+int begin_batch_launch(BatchStatus* b, cudaStream_t stream);
 // Polls of a first wait before a thread block gives up (default 2^20; the
 // drain of copies still in flight after a give-up always uses the default).
 constexpr int kDefaultWaitPolls = 1 << 20;

@@ -491,7 +491,7 @@ int launch_tma(const void* inp, const void* coeff, void* out, int64_t ni, int64_
     const int64_t gx = ceil_div(ni, TX), gy = ceil_div(nj, ty), gz = ceil_div(nk, kper);
     SB_CHECK(gy <= p->max_grid_y && gz <= p->max_grid_z, SB_ERR_INVALID, "hdiff grid too large");
     int* status = nullptr;
-    const int rc = status_word(&status);
+    const int rc = status_word(stream, &status);
     if (rc) return rc;
     t_tma_used = true;
     kernel<<<dim3((unsigned)gx, (unsigned)gy, (unsigned)gz), dim3(TX, NTY), smem, stream>>>(
@@ -744,10 +744,10 @@ extern "C" int sb_hdiff(int storage, int compute, const void* inp, const void* c
         if (time_s) *time_s = 0.0;
         return SB_OK;
     }
-    // a give-up of an earlier launch is reported before anything new runs
-    rc = take_wait_status();
-    if (rc) return rc;
     cudaStream_t s = (cudaStream_t)stream;
+    // a give-up of an earlier launch on the stream is reported before anything new runs
+    rc = take_stream_status(s);
+    if (rc) return rc;
     t_tma_used = false;
     rc = timed(s, time_s, [&]() {
         if (storage == SB_F64 && compute == SB_F64)
@@ -764,6 +764,6 @@ extern "C" int sb_hdiff(int storage, int compute, const void* inp, const void* c
             return launch_typed<bf16, float>(inp, coeff, out, ni, nj, nk, si, sj, sk, tune, s);
         return fail(SB_ERR_UNSUPPORTED, "unsupported storage/compute combination (%d, %d)", storage, compute);
     });
-    if (rc == SB_OK && time_s && t_tma_used) rc = take_wait_status();
+    if (rc == SB_OK && time_s && t_tma_used) rc = take_stream_status(s);
     return rc;
 }

@@ -53,25 +53,95 @@ int device_props(const DeviceProps** out) {
 }
 
 namespace {
-std::once_flag g_status_once;
-int* g_status = nullptr;  // host address == device address (unified addressing)
-cudaError_t g_status_error = cudaSuccess;
+constexpr int kStatusWords = 1024;
+struct StreamStatus {
+    std::atomic<cudaStream_t> stream;
+    std::atomic<bool> hidden;
+};
+// Every launching call looks its stream up, so that takes no lock (two, and a
+// cudaGetDevice each, made a 15 us call 1 us longer); the mutex orders changes
+// of the table and the list of batches.
+std::mutex g_status_mutex;
+int* g_status = nullptr;  // kStatusWords words; host address == device address (unified addressing)
+StreamStatus g_streams[kStatusWords];  // entry n has word n; entry 0: streams beyond the table
+std::atomic<int> g_nstreams{1};        // entries ever used
+BatchStatus* g_batches = nullptr;
+std::atomic<int> g_nbatches{0};
 std::atomic<int> g_wait_polls{kDefaultWaitPolls};
+char g_free_mark, g_lost_mark;
+// entries of no stream: to be used again, or with a launch that may still set the word
+const cudaStream_t kFree = (cudaStream_t)&g_free_mark, kLost = (cudaStream_t)&g_lost_mark;
+
+int find_stream(cudaStream_t s) {
+    const int count = g_nstreams.load(std::memory_order_acquire);
+    for (int n = 1; n < count; ++n)
+        if (g_streams[n].stream.load(std::memory_order_acquire) == s) return n;
+    return 0;
+}
+// with the mutex held; 0: the table is full
+int add_stream(cudaStream_t s) {
+    int n = find_stream(s);
+    if (n) return n;
+    n = find_stream(kFree);
+    const int count = g_nstreams.load();
+    if (!n && count == kStatusWords) return 0;
+    if (!n) n = count;
+    g_streams[n].hidden = false;
+    g_streams[n].stream = s;
+    if (n == count) g_nstreams.store(count + 1, std::memory_order_release);
+    return n;
+}
+bool take_word(int* w) { return __atomic_load_n(w, __ATOMIC_ACQUIRE) && __atomic_exchange_n(w, 0, __ATOMIC_ACQ_REL); }
+
+// with the mutex held
+int allocate_words() {
+    if (g_status) return SB_OK;
+    // another thread's capture must not see the allocation
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    void* p = nullptr;
+    const cudaError_t e = cudaHostAlloc(&p, kStatusWords * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return fail(SB_ERR_CUDA, "cudaHostAlloc of the wait-status words failed: %s", cudaGetErrorString(e));
+    }
+    memset(p, 0, kStatusWords * sizeof(int));
+    __atomic_store_n(&g_status, static_cast<int*>(p), __ATOMIC_RELEASE);
+    return SB_OK;
+}
+
+int gave_up() {
+    return fail(SB_ERR_TIMEOUT,
+                "a thread block of an earlier launch gave up waiting for its tensor copies: that launch's "
+                "output is incomplete");
+}
+
+bool take_stream_words(cudaStream_t stream) {
+    int* const words = __atomic_load_n(&g_status, __ATOMIC_ACQUIRE);
+    const int n = words ? find_stream(stream) : 0;
+    return n && take_word(words + n);
+}
+// with the mutex held
+bool take_batch_words(cudaStream_t stream) {
+    bool set = false;
+    for (BatchStatus* b = g_batches; b; b = b->next)
+        if (b->launched && b->stream == stream) set |= take_word(b->word);
+    return set;
+}
 }  // namespace
 
-int status_word(int** device_ptr) {
-    std::call_once(g_status_once, [] {
-        void* p = nullptr;
-        g_status_error = cudaHostAlloc(&p, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable);
-        if (g_status_error == cudaSuccess) {
-            g_status = static_cast<int*>(p);
-            __atomic_store_n(g_status, 0, __ATOMIC_RELEASE);
-        }
-    });
-    if (!g_status)
-        return fail(SB_ERR_CUDA, "cudaHostAlloc of the wait-status word failed: %s",
-                    cudaGetErrorString(g_status_error));
-    *device_ptr = g_status;
+int status_word(cudaStream_t stream, int** device_ptr) {
+    int* words = __atomic_load_n(&g_status, __ATOMIC_ACQUIRE);
+    int n = words ? find_stream(stream) : 0;
+    if (!n) {
+        std::lock_guard<std::mutex> lock(g_status_mutex);
+        const int rc = allocate_words();
+        if (rc) return rc;
+        words = g_status;
+        n = add_stream(stream);
+    }
+    *device_ptr = words + n;
     return SB_OK;
 }
 
@@ -85,11 +155,69 @@ bool status_ready(cudaStream_t stream) {
     return cs == cudaStreamCaptureStatusNone;
 }
 
-int take_wait_status() {
-    if (!g_status || !__atomic_exchange_n(g_status, 0, __ATOMIC_ACQ_REL)) return SB_OK;
-    return fail(SB_ERR_TIMEOUT,
-                "a thread block of an earlier launch gave up waiting for its tensor copies: that launch's "
-                "output is incomplete");
+int take_stream_status(cudaStream_t stream) {
+    bool set = take_stream_words(stream);
+    if (g_nbatches.load(std::memory_order_acquire)) {
+        std::lock_guard<std::mutex> lock(g_status_mutex);
+        set |= take_batch_words(stream);
+    }
+    return set ? gave_up() : SB_OK;
+}
+
+int take_status() {
+    std::lock_guard<std::mutex> lock(g_status_mutex);
+    bool set = false;
+    if (g_status)
+        for (int n = 0; n < g_nstreams; ++n)
+            if (!g_streams[n].hidden) set |= take_word(g_status + n);
+    for (BatchStatus* b = g_batches; b; b = b->next)
+        if (!(b->launched && g_streams[find_stream(b->stream)].hidden)) set |= take_word(b->word);
+    return set ? gave_up() : SB_OK;
+}
+
+int make_stream_private(cudaStream_t stream) {
+    std::lock_guard<std::mutex> lock(g_status_mutex);
+    const int n = add_stream(stream);
+    SB_CHECK(n, SB_ERR_NOMEM, "no wait-status word left for another stream (%d in use)", kStatusWords);
+    g_streams[n].hidden = true;
+    return SB_OK;
+}
+
+void forget_stream(cudaStream_t stream) {
+    const bool idle = cudaStreamQuery(stream) == cudaSuccess;
+    if (!idle) cudaGetLastError();
+    std::lock_guard<std::mutex> lock(g_status_mutex);
+    const int n = find_stream(stream);
+    if (!n) return;
+    if (g_status && take_word(g_status + n)) __atomic_store_n(g_status, 1, __ATOMIC_RELEASE);
+    g_streams[n].hidden = false;
+    g_streams[n].stream = idle ? kFree : kLost;
+}
+
+void list_batch_status(BatchStatus* b) {
+    std::lock_guard<std::mutex> lock(g_status_mutex);
+    b->next = g_batches;
+    if (g_batches) g_batches->prev = b;
+    g_batches = b;
+    ++g_nbatches;
+}
+
+void unlist_batch_status(BatchStatus* b) {
+    std::lock_guard<std::mutex> lock(g_status_mutex);
+    if (take_word(b->word) && allocate_words() == SB_OK) __atomic_store_n(g_status, 1, __ATOMIC_RELEASE);
+    if (b->prev) b->prev->next = b->next;
+    else g_batches = b->next;
+    if (b->next) b->next->prev = b->prev;
+    --g_nbatches;
+}
+
+int begin_batch_launch(BatchStatus* b, cudaStream_t stream) {
+    std::lock_guard<std::mutex> lock(g_status_mutex);
+    const bool own = take_word(b->word), plain = take_stream_words(stream), batches = take_batch_words(stream);
+    if (own || plain || batches) return gave_up();
+    b->stream = stream;
+    b->launched = true;
+    return SB_OK;
 }
 
 int wait_polls() { return g_wait_polls.load(std::memory_order_relaxed); }
@@ -396,10 +524,10 @@ int sb_device_info(int device, char* name, int name_len, int* sm_count, int* cc_
 
 int sb_synchronize(void) {
     SB_CUDA(cudaDeviceSynchronize());
-    return take_wait_status();
+    return take_status();
 }
 
-int sb_kernel_status(void) { return take_wait_status(); }
+int sb_kernel_status(void) { return take_status(); }
 
 int sb_debug_wait_limit(int polls) {
     SB_CHECK(polls >= -1, SB_ERR_INVALID, "polls must be >= -1");
@@ -498,13 +626,16 @@ int sb_stream_create(void** stream) {
 }
 
 int sb_stream_destroy(void* stream) {
-    if (stream) SB_CUDA(cudaStreamDestroy((cudaStream_t)stream));
+    if (stream) {
+        forget_stream((cudaStream_t)stream);
+        SB_CUDA(cudaStreamDestroy((cudaStream_t)stream));
+    }
     return SB_OK;
 }
 
 int sb_stream_synchronize(void* stream) {
     SB_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
-    return take_wait_status();
+    return take_status();
 }
 
 int sb_event_create(void** event) {
@@ -527,7 +658,7 @@ int sb_event_record(void* event, void* stream) {
 
 int sb_event_synchronize(void* event) {
     SB_CUDA(cudaEventSynchronize((cudaEvent_t)event));
-    return take_wait_status();
+    return take_status();
 }
 
 int sb_event_elapsed(void* start, void* stop, double* seconds) {

@@ -620,8 +620,10 @@ int launch_tma_maps(const DeviceProps* p, cudaStream_t stream, const TmemCompone
     a.warp_bytes = shape.warp_bytes;
     // at least 120 KB: one block per SM, so the 512-column allocation is free
     const size_t smem = std::max<size_t>(B::ring_offset(shape.warps) + (size_t)shape.warps * shape.warp_bytes, 120 * 1024);
-    const int rc = status_word(&a.status);
-    if (rc) return rc;
+    if (status_word(stream, &a.status)) {
+        clear_error();
+        return SB_ERR_UNSUPPORTED;  // the forms without waits need no word
+    }
     auto kernel = vadv_tma_kernel<S, R, NC>;
     SB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int64_t grid = std::min<int64_t>(p->sm_count, ceil_div(ngroups, (int64_t)shape.warps));
@@ -933,10 +935,10 @@ extern "C" int sb_vadv3(int storage, int compute, const void* const* stage, cons
         return SB_OK;
     }
     SB_CHECK(nk >= 2, SB_ERR_INVALID, "vertical advection needs at least 2 levels (nk = %lld)", (long long)nk);
-    // a give-up of an earlier launch is reported before anything new runs
-    rc = take_wait_status();
-    if (rc) return rc;
     cudaStream_t s = (cudaStream_t)stream;
+    // a give-up of an earlier launch on the stream is reported before anything new runs
+    rc = take_stream_status(s);
+    if (rc) return rc;
     t_waits = false;
     rc = timed(s, time_s, [&]() {
         if (storage == SB_F64 && compute == SB_F64)
@@ -949,7 +951,7 @@ extern "C" int sb_vadv3(int storage, int compute, const void* const* stage, cons
             return launch_typed3<float, double>(stage, pos, tens, tensstage, wcon, out, ccol, dcol, ni, nj, nk, si, sj, sk, tune, s);
         return launch_typed3<bf16, float>(stage, pos, tens, tensstage, wcon, out, ccol, dcol, ni, nj, nk, si, sj, sk, tune, s);
     });
-    if (rc == SB_OK && time_s && t_waits) rc = take_wait_status();
+    if (rc == SB_OK && time_s && t_waits) rc = take_stream_status(s);
     return rc;
 }
 
@@ -973,10 +975,10 @@ extern "C" int sb_vadv(int storage, int compute, const void* stage, const void* 
     }
     SB_CHECK(nk >= 2, SB_ERR_INVALID, "vertical advection needs at least 2 levels (nk = %lld)", (long long)nk);
     const int64_t wsh = (int64_t)wshift_i * si + (int64_t)wshift_j * sj;
-    // a give-up of an earlier launch is reported before anything new runs
-    rc = take_wait_status();
-    if (rc) return rc;
     cudaStream_t s = (cudaStream_t)stream;
+    // a give-up of an earlier launch on the stream is reported before anything new runs
+    rc = take_stream_status(s);
+    if (rc) return rc;
     t_waits = false;
     rc = timed(s, time_s, [&]() {
         if (storage == SB_F64 && compute == SB_F64)
@@ -991,6 +993,6 @@ extern "C" int sb_vadv(int storage, int compute, const void* stage, const void* 
             return launch_typed<bf16, float>(stage, pos, tens, tensstage, wcon, out, ccol, dcol, ni, nj, nk, si, sj, sk, wsh, tune, s);
         return fail(SB_ERR_UNSUPPORTED, "unsupported storage/compute combination (%d, %d)", storage, compute);
     });
-    if (rc == SB_OK && time_s && t_waits) rc = take_wait_status();
+    if (rc == SB_OK && time_s && t_waits) rc = take_stream_status(s);
     return rc;
 }

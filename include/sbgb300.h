@@ -163,8 +163,8 @@ int sb_synchronize(void);
  * streams are not affected), sb_synchronize, sb_stream_synchronize,
  * sb_event_synchronize (each reports any stream's), or sb_kernel_status.  A
  * launch captured into the caller's own graph counts as one of the stream it
- * was captured from.  No reference counterpart (its kernels do not wait on the
- * device).
+ * was captured from; a server's launches are reported by sb_server_step only.
+ * No reference counterpart (its kernels do not wait on the device).
  * sb_kernel_status: SB_ERR_TIMEOUT if a launch has given up since the last
  * report, else SB_OK; does not synchronise.
  * sb_debug_wait_limit: testing aid, the polls of each first wait (0: give up
@@ -401,7 +401,11 @@ int sb_arena_destroy(sb_arena* arena);
  * sb_server_release; sb_server_query reports the times of a request the
  * server still holds.  simulate = 1 makes no CUDA call (scheduling tests;
  * sb_server_debug_complete finishes the in-flight slots, sb_server_debug_launches
- * lists the launches as (storage, requests)).  One thread per server.        */
+ * lists the launches as (storage, requests)).  One thread per server.
+ * A step that finds that a kernel gave up a bounded wait returns
+ * SB_ERR_TIMEOUT: none of the requests launched with it is completed, and the
+ * next step launches them again.  Requests whose launch fails stay queued, and
+ * every step returns the error until they can be launched.                    */
 typedef struct sb_server sb_server;
 typedef struct sb_server_config {
     uint64_t budget_bytes;

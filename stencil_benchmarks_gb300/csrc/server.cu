@@ -5,7 +5,9 @@
 // One sb_server_step(now):
 //   1. poll: every slot whose completion event has fired retires its requests
 //      (completed = now) and returns their fields to the arena, except the
-//      kept ones;
+//      kept ones.  Where one of its kernels gave up a bounded wait, outputs are
+//      incomplete: its requests go back to the head of their queue, to be
+//      launched again, and the step returns SB_ERR_TIMEOUT;
 //   2. admit: waiting requests, in arrival order, get their fields from the
 //      budget-capped arena (one device region allocated at creation, carved
 //      by sb_arena: no cudaMalloc per request); the inputs of everything
@@ -14,7 +16,8 @@
 //   3. dispatch: for every precision form with admitted requests and a free
 //      slot, up to max_batch of them are packed into that slot's sb_batch and
 //      launched (one graph replay) on the slot's stream after the fill, or,
-//      in plain mode, launched one sb_hdiff / sb_vadv each.
+//      in plain mode, launched one sb_hdiff / sb_vadv each.  Requests whose
+//      launch fails stay at the head of their queue.
 // Several slots per form are in flight at once: requests that arrive while
 // others run are admitted as memory frees up and overlap on the device.
 //
@@ -80,6 +83,7 @@ struct Slot {
     cudaEvent_t done = nullptr;
     std::vector<Req*> reqs;
     bool busy = false;
+    bool gave_up = false;  // a launch that was refused reported an earlier one of this slot
     bool sim_done = false;
 };
 
@@ -128,7 +132,10 @@ struct sb_server {
             for (auto& forms : slots)
                 for (auto& s : forms) {
                     if (s.batch) sb_batch_destroy(s.batch);
-                    if (s.stream) cudaStreamDestroy(s.stream);
+                    if (s.stream) {
+                        forget_stream(s.stream);
+                        cudaStreamDestroy(s.stream);
+                    }
                     if (s.done) cudaEventDestroy(s.done);
                 }
             for (auto& e : fill_events)
@@ -159,6 +166,7 @@ struct sb_server {
     }
 
     int poll(double now) {
+        int status = SB_OK;
         for (int form = 0; form < kForms; ++form) {
             for (auto& s : slots[form]) {
                 if (!s.busy) continue;
@@ -168,6 +176,16 @@ struct sb_server {
                     const cudaError_t e = cudaEventQuery(s.done);
                     if (e == cudaErrorNotReady) continue;
                     if (e != cudaSuccess) return fail(SB_ERR_CUDA, "server: %s", cudaGetErrorString(e));
+                    if (take_stream_status(s.stream) != SB_OK) s.gave_up = true;
+                }
+                if (s.gave_up) {
+                    status = fail(SB_ERR_TIMEOUT,
+                                  "server: a kernel gave up waiting for its tensor copies; the %d requests launched "
+                                  "with it run again", (int)s.reqs.size());
+                    for (Req* q : s.reqs) q->launched = -1.0;
+                    ready[form].insert(ready[form].begin(), s.reqs.begin(), s.reqs.end());
+                    retire(s);
+                    continue;
                 }
                 for (Req* q : s.reqs) {
                     q->completed = now;
@@ -176,13 +194,16 @@ struct sb_server {
                     completed.push_back(sb_completion{q->r.id, q->r.arrival, q->admitted, q->launched, q->completed});
                     if (!q->kept) reqs.erase(q->r.id);
                 }
-                inflight -= (int64_t)s.reqs.size();
-                s.reqs.clear();
-                s.busy = false;
-                s.sim_done = false;
+                retire(s);
             }
         }
-        return SB_OK;
+        return status;
+    }
+
+    void retire(Slot& s) {
+        inflight -= (int64_t)s.reqs.size();
+        s.reqs.clear();
+        s.busy = s.gave_up = s.sim_done = false;
     }
 
     int admit(double now) {
@@ -267,6 +288,32 @@ struct sb_server {
                        d.nj, d.nk, d.si, d.sj, d.sk, 1, 0, nullptr, stream, nullptr);
     }
 
+    // Launch the slot's requests; `launched` is how many of them are on their way.
+    int launch(Slot& slot, int form, int& launched) {
+        launched = 0;
+        if (fill_last >= 0) SB_CUDA(cudaStreamWaitEvent(slot.stream, fill_events[fill_last], 0));
+        int rc = SB_OK;
+        if (cfg.mode == 0) {
+            doms.clear();
+            for (const Req* q : slot.reqs) doms.push_back(domain_of(q));
+            rc = sb_batch_set(slot.batch, doms.data(), (int)doms.size());
+            if (rc == SB_OK) rc = sb_batch_launch(slot.batch, slot.stream, nullptr);
+            if (rc == SB_OK) launched = (int)slot.reqs.size();
+        } else {
+            for (const Req* q : slot.reqs) {
+                rc = launch_one(q, form, slot.stream);
+                if (rc) break;
+                ++launched;
+            }
+        }
+        if (rc == SB_ERR_TIMEOUT && launched) {  // of one of the launches before it
+            slot.gave_up = true;
+            rc = SB_OK;
+        }
+        if (launched) SB_CUDA(cudaEventRecord(slot.done, slot.stream));
+        return rc;
+    }
+
     int dispatch(double now) {
         for (int form = 0; form < kForms; ++form) {
             auto& queue = ready[form];
@@ -280,28 +327,19 @@ struct sb_server {
                 if (!slot) break;
                 const int n = (int)std::min<size_t>((size_t)cfg.max_batch, queue.size());
                 slot->reqs.assign(queue.begin(), queue.begin() + n);
-                queue.erase(queue.begin(), queue.begin() + n);
+                int launched = n, rc = SB_OK;
                 if (sim()) {
                     launch_log.push_back(sb_server_launch{storage_of(form), n});
                 } else {
-                    if (fill_last >= 0) SB_CUDA(cudaStreamWaitEvent(slot->stream, fill_events[fill_last], 0));
-                    if (cfg.mode == 0) {
-                        doms.clear();
-                        for (const Req* q : slot->reqs) doms.push_back(domain_of(q));
-                        int rc = sb_batch_set(slot->batch, doms.data(), n);
-                        if (rc == SB_OK) rc = sb_batch_launch(slot->batch, slot->stream, nullptr);
-                        if (rc) return rc;
-                    } else {
-                        for (const Req* q : slot->reqs) {
-                            const int rc = launch_one(q, form, slot->stream);
-                            if (rc) return rc;
-                        }
-                    }
-                    SB_CUDA(cudaEventRecord(slot->done, slot->stream));
+                    rc = launch(*slot, form, launched);
                 }
+                // what was not launched stays in the queue
+                slot->reqs.resize(launched);
+                queue.erase(queue.begin(), queue.begin() + launched);
                 for (Req* q : slot->reqs) q->launched = now;
-                inflight += n;
-                slot->busy = true;
+                inflight += launched;
+                slot->busy = launched > 0;
+                if (rc) return rc;
             }
         }
         return SB_OK;
@@ -347,6 +385,8 @@ int sb_server_create(sb_server** out, const sb_server_config* cfg_in) {
         if (s->sim()) continue;
         for (auto& slot : s->slots[form]) {
             SB_CUDA(cudaStreamCreateWithFlags(&slot.stream, cudaStreamNonBlocking));
+            rc = make_stream_private(slot.stream);  // poll has to see every give-up
+            if (rc) return rc;
             SB_CUDA(cudaEventCreateWithFlags(&slot.done, cudaEventDisableTiming));
             if (cfg.mode == 0) {
                 const int storage = s->storage_of(form);

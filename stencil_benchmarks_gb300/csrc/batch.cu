@@ -588,13 +588,21 @@ int capture_graph(sb_batch* b) {
         cudaGraphDestroy(b->graph);
         b->graph = nullptr;
     }
+    const DeviceProps* p;
+    const int prc = device_props(&p);
+    if (prc) return prc;
     Kinds k;
     SB_CHECK(pick_kinds(b->storage, b->compute, b->idx64, &k), SB_ERR_UNSUPPORTED, "unsupported form");
     auto vadv_run = b->vadv_block == 64 ? k.vadv64 : k.vadv32;
     const void* vadv_fn = b->vadv_block == 64 ? k.vadv64_fn : k.vadv32_fn;
     for (int q = 0; q < kBuckets; ++q) {
-        if (b->vadv_smem[q] > 48 * 1024)
-            SB_CUDA(cudaFuncSetAttribute(vadv_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->vadv_smem[q]));
+        if (b->vadv_smem[q] > 48 * 1024) {
+            cudaFuncAttributes fa;
+            SB_CUDA(cudaFuncGetAttributes(&fa, vadv_fn));
+            const int rc = allow_smem(vadv_fn, p, fa.sharedSizeBytes);
+            if (rc) return rc;
+            break;
+        }
     }
     TmaBatch ta{};
     size_t tma_smem = 0;
@@ -603,10 +611,13 @@ int capture_graph(sb_batch* b) {
         const TmaShape& sh = b->tma_shapes[b->use_tma];
         ta = {sh.nt, sh.stages, c.stage_bytes(b->use_tma >= kTmaClasses), sh.warp_bytes, wait_polls(), b->status.word};
         tma_smem = std::max<size_t>(c.ring_offset(sh.warps) + (size_t)sh.warps * sh.warp_bytes, 120 * 1024);
-        SB_CUDA(cudaFuncSetAttribute(c.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tma_smem));
+        const int rc = allow_smem(c.fn, p);
+        if (rc) return rc;
         b->graph_polls = ta.polls;
-    } else if (b->use_tmem)
-        SB_CUDA(cudaFuncSetAttribute(k.vadv_tmem_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->tmem_smem));
+    } else if (b->use_tmem) {
+        const int rc = allow_smem(k.vadv_tmem_fn, p);
+        if (rc) return rc;
+    }
     cudaStream_t s0 = b->streams[0];
     SB_CUDA(cudaStreamBeginCapture(s0, cudaStreamCaptureModeThreadLocal));
     cudaMemcpyAsync(b->dev_table, b->host_table, table_bytes(b->max_domains), cudaMemcpyHostToDevice, s0);

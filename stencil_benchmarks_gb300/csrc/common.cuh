@@ -6,6 +6,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <cstdio>
 
@@ -469,6 +470,25 @@ __device__ __forceinline__ void st_vec(S* p, const C (&v)[V]) {
 // ---------------------------------------------------------------------------
 // launch helpers
 // ---------------------------------------------------------------------------
+
+// Let a kernel use up to all of a block's shared memory.  Never a call's own
+// size: the limit is the kernel's, and a thread with a smaller call could lower
+// it between another one's setting and its launch, which then fails.
+// static_bytes: what the kernel declares besides the dynamic part.
+inline int allow_smem(const void* kernel, const DeviceProps* p, size_t static_bytes = 0) {
+    SB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, p->smem_optin - (int)static_bytes));
+    return SB_OK;
+}
+// The same once per device, for the calls of one kernel each (0.5 of 15 us of a small vadv call).
+template <auto KERNEL>
+int allow_smem(const DeviceProps* p) {
+    static std::atomic<uint64_t> devices{0};
+    const uint64_t bit = p->device < 64 ? 1ull << p->device : 0;
+    if (devices.load(std::memory_order_acquire) & bit) return SB_OK;
+    const int rc = allow_smem((const void*)KERNEL, p);
+    if (rc == SB_OK) devices.fetch_or(bit, std::memory_order_release);
+    return rc;
+}
 
 // Run `launch()` on `stream`; with `time_s` non-NULL time it with CUDA events
 // (reference: stencils/cuda_hip/templates/base.j2:145-190).

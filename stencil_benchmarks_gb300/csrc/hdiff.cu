@@ -275,7 +275,10 @@ int launch_tile(const void* inp, const void* coeff, void* out, int64_t ni, int64
              "hdiff tile %dx%d needs %zu bytes of shared memory (device limit %d)", TX, ty, smem,
              p->smem_optin);
     auto kernel = hdiff_tile_kernel<S, C, TX, NTY>;
-    if (smem > 48 * 1024) SB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024) {
+        const int arc = allow_smem<hdiff_tile_kernel<S, C, TX, NTY>>(p);
+        if (arc) return arc;
+    }
     const int64_t gx = ceil_div(ni, TX), gy = ceil_div(nj, ty), gz = ceil_div(nk, kper);
     SB_CHECK(gy <= p->max_grid_y && gz <= p->max_grid_z, SB_ERR_INVALID, "hdiff grid too large");
     kernel<<<dim3((unsigned)gx, (unsigned)gy, (unsigned)gz), dim3(TX, NTY), smem, stream>>>(
@@ -487,7 +490,10 @@ int launch_tma(const void* inp, const void* coeff, void* out, int64_t ni, int64_
     SB_CHECK((int64_t)smem <= p->smem_optin, SB_ERR_INVALID, "hdiff TMA tile %dx%d needs %zu bytes of shared memory",
              TX, ty, smem);
     auto kernel = hdiff_tma_kernel<S, C, TX, NTY, PL>;
-    if (smem > 48 * 1024) SB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024) {
+        const int arc = allow_smem<hdiff_tma_kernel<S, C, TX, NTY, PL>>(p);
+        if (arc) return arc;
+    }
     const int64_t gx = ceil_div(ni, TX), gy = ceil_div(nj, ty), gz = ceil_div(nk, kper);
     SB_CHECK(gy <= p->max_grid_y && gz <= p->max_grid_z, SB_ERR_INVALID, "hdiff grid too large");
     int* status = nullptr;

@@ -208,11 +208,14 @@ __global__ void __launch_bounds__(32 * W)
 }
 
 template <class S, class C, bool GLOBAL, int D>
-int launch_one(dim3 grid, dim3 block, size_t smem, cudaStream_t stream, const void* stage, const void* pos,
+int launch_one(const DeviceProps* p, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, const void* stage, const void* pos,
                const void* tens, const void* tensstage, const void* wcon, void* out, void* ccol, void* dcol,
                int64_t ni, int64_t nj, int64_t nk, int64_t si, int64_t sj, int64_t sk, int64_t wsh) {
     auto kernel = vadv_kernel<S, C, GLOBAL, D>;
-    if (smem > 48 * 1024) SB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024) {
+        const int rc = allow_smem<vadv_kernel<S, C, GLOBAL, D>>(p);
+        if (rc) return rc;
+    }
     kernel<<<grid, block, smem, stream>>>((const S*)stage, (const S*)pos, (const S*)tens, (const S*)tensstage,
                                           (const S*)wcon, (S*)out, (C*)ccol, (C*)dcol, (int)ni, (int)nj, (int)nk,
                                           si, sj, sk, wsh);
@@ -220,15 +223,15 @@ int launch_one(dim3 grid, dim3 block, size_t smem, cudaStream_t stream, const vo
 }
 
 template <class S, class C, bool GLOBAL>
-int launch_depth(int depth, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, const void* stage,
+int launch_depth(int depth, const DeviceProps* p, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, const void* stage,
                  const void* pos, const void* tens, const void* tensstage, const void* wcon, void* out,
                  void* ccol, void* dcol, int64_t ni, int64_t nj, int64_t nk, int64_t si, int64_t sj,
                  int64_t sk, int64_t wsh) {
     switch (depth) {
-        case 1: return launch_one<S, C, GLOBAL, 1>(grid, block, smem, stream, stage, pos, tens, tensstage, wcon, out, ccol, dcol, ni, nj, nk, si, sj, sk, wsh);
-        case 2: return launch_one<S, C, GLOBAL, 2>(grid, block, smem, stream, stage, pos, tens, tensstage, wcon, out, ccol, dcol, ni, nj, nk, si, sj, sk, wsh);
-        case 4: return launch_one<S, C, GLOBAL, 4>(grid, block, smem, stream, stage, pos, tens, tensstage, wcon, out, ccol, dcol, ni, nj, nk, si, sj, sk, wsh);
-        case 8: return launch_one<S, C, GLOBAL, 8>(grid, block, smem, stream, stage, pos, tens, tensstage, wcon, out, ccol, dcol, ni, nj, nk, si, sj, sk, wsh);
+        case 1: return launch_one<S, C, GLOBAL, 1>(p, grid, block, smem, stream, stage, pos, tens, tensstage, wcon, out, ccol, dcol, ni, nj, nk, si, sj, sk, wsh);
+        case 2: return launch_one<S, C, GLOBAL, 2>(p, grid, block, smem, stream, stage, pos, tens, tensstage, wcon, out, ccol, dcol, ni, nj, nk, si, sj, sk, wsh);
+        case 4: return launch_one<S, C, GLOBAL, 4>(p, grid, block, smem, stream, stage, pos, tens, tensstage, wcon, out, ccol, dcol, ni, nj, nk, si, sj, sk, wsh);
+        case 8: return launch_one<S, C, GLOBAL, 8>(p, grid, block, smem, stream, stage, pos, tens, tensstage, wcon, out, ccol, dcol, ni, nj, nk, si, sj, sk, wsh);
     }
     return fail(SB_ERR_INVALID, "vadv prefetch depth (unroll) must be 1, 2, 4 or 8 (got %d)", depth);
 }
@@ -243,11 +246,14 @@ size_t async_smem(int64_t nk, int bt, int depth, int* ring_offset) {
 }
 
 template <class S, class C, int BT, int D, class P>
-int launch_async_one(dim3 grid, size_t smem, int ring_offset, cudaStream_t stream, const void* stage,
+int launch_async_one(const DeviceProps* p, dim3 grid, size_t smem, int ring_offset, cudaStream_t stream, const void* stage,
                      const void* pos, const void* tens, const void* tensstage, const void* wcon, void* out,
                      int64_t ni, int64_t nj, int64_t nk, int64_t si, int64_t sj, int64_t sk, int64_t wsh) {
     auto kernel = vadv_async_kernel<S, C, BT, D, P>;
-    if (smem > 48 * 1024) SB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024) {
+        const int rc = allow_smem<vadv_async_kernel<S, C, BT, D, P>>(p);
+        if (rc) return rc;
+    }
     kernel<<<grid, BT, smem, stream>>>((const S*)stage, (const S*)pos, (const S*)tens, (const S*)tensstage,
                                        (const S*)wcon, (S*)out, (int)ni, (int)nj, (int)nk, (int)si, (int)sj,
                                        (int)sk, (int)wsh, ring_offset);
@@ -274,7 +280,7 @@ int launch_async(int bx, int by, int depth, const DeviceProps* p, cudaStream_t s
     const dim3 grid((unsigned)ceil_div(ni, bx), (unsigned)nj);
 #define SB_VADV_ASYNC(BTV, DV)                                                                              \
     if (bx == BTV && depth == DV)                                                                           \
-        return launch_async_one<S, C, BTV, DV, P>(grid, smem, ring_offset, stream, stage, pos, tens, tensstage, \
+        return launch_async_one<S, C, BTV, DV, P>(p, grid, smem, ring_offset, stream, stage, pos, tens, tensstage, \
                                                wcon, out, ni, nj, nk, si, sj, sk, wsh);
     SB_VADV_ASYNC(32, 4)
     SB_VADV_ASYNC(32, 8)
@@ -292,7 +298,10 @@ int launch_slab_one(int blocks_per_sm, const DeviceProps* p, cudaStream_t stream
                     int64_t wsh) {
     auto kernel = vadv_slab_kernel<S, C, BT, D, PL>;
     const size_t smem = (size_t)(D + 1) * 6 * BT * sizeof(typename RingOf<S>::T);
-    if (smem > 48 * 1024) SB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024) {
+        const int rc = allow_smem<vadv_slab_kernel<S, C, BT, D, PL>>(p);
+        if (rc) return rc;
+    }
     int fit = 0;
     SB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kernel, BT, smem));
     int per_sm = std::max(1, fit);
@@ -393,7 +402,10 @@ int launch_wslab_one(int blocks_per_sm, const DeviceProps* p, cudaStream_t strea
     constexpr int BT = 32 * W;
     auto kernel = vadv_wslab_kernel<S, C, W, D>;
     const size_t smem = (size_t)W * WarpRing<S, C, D>::BYTES;
-    if (smem > 48 * 1024) SB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024) {
+        const int rc = allow_smem<vadv_wslab_kernel<S, C, W, D>>(p);
+        if (rc) return rc;
+    }
     int fit = 0;
     SB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kernel, BT, smem));
     int per_sm = std::max(1, fit);
@@ -509,7 +521,8 @@ int launch_tmem_one(int g4, int cpw, bool sa, const DeviceProps* p, cudaStream_t
     // at least 120 KB: one block per SM, so the 512-column allocation is free
     const size_t smem = std::max<size_t>(16 + (size_t)nwarps * WarpRing<S, float, D>::BYTES, 120 * 1024);
     if ((int64_t)smem > p->smem_optin) return SB_ERR_UNSUPPORTED;
-    SB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int rc = allow_smem((const void*)kernel, p);
+    if (rc) return rc;
     const int64_t ngroups = ceil_div(ni, (int64_t)32) * nj;
     const int64_t grid = std::min<int64_t>(p->sm_count, ceil_div(ngroups, (int64_t)nwarps));
     kernel<<<(unsigned)grid, 32 * nwarps, smem, stream>>>(comps, (const S*)wcon, (int)ni, (int)nj, (int)nk,
@@ -625,7 +638,8 @@ int launch_tma_maps(const DeviceProps* p, cudaStream_t stream, const TmemCompone
         return SB_ERR_UNSUPPORTED;  // the forms without waits need no word
     }
     auto kernel = vadv_tma_kernel<S, R, NC>;
-    SB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int rc = allow_smem<vadv_tma_kernel<S, R, NC>>(p);
+    if (rc) return rc;
     const int64_t grid = std::min<int64_t>(p->sm_count, ceil_div(ngroups, (int64_t)shape.warps));
     t_waits = true;
     kernel<<<(unsigned)grid, (unsigned)(32 * shape.warps), smem, stream>>>(a);
@@ -803,11 +817,11 @@ int launch_typed(const void* stage, const void* pos, const void* tens, const voi
                  "vadv: %lld levels x %d columns need %zu bytes of shared memory (limit %d); "
                  "use fewer threads per block or the GLOBAL variant with ccol/dcol scratch",
                  (long long)nk, bx * by, smem, p->smem_optin);
-        return launch_depth<S, C, false>(depth, grid, block, smem, stream, stage, pos, tens, tensstage, wcon, out,
+        return launch_depth<S, C, false>(depth, p, grid, block, smem, stream, stage, pos, tens, tensstage, wcon, out,
                                          nullptr, nullptr, ni, nj, nk, si, sj, sk, wsh);
     }
     SB_CHECK(can_global, SB_ERR_INVALID, "vadv GLOBAL variant needs ccol/dcol scratch fields of the compute type");
-    return launch_depth<S, C, true>(depth, grid, block, 0, stream, stage, pos, tens, tensstage, wcon, out,
+    return launch_depth<S, C, true>(depth, p, grid, block, 0, stream, stage, pos, tens, tensstage, wcon, out,
                                     ccol, dcol, ni, nj, nk, si, sj, sk, wsh);
 }
 

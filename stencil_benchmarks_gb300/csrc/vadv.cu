@@ -856,11 +856,12 @@ int launch_typed3(const void* const* stage, const void* const* pos, const void* 
                 comps.wsh[c] = (int)wsh[c];
             }
             comps.nc = 3;
-            // the TMA form reads a component's fields while the one before it is still being written
+            // the TMA form reads a component's fields while the one before it is still being
+            // written, and wcon of other columns until the last component is done
             bool apart = true;
             for (int c = 0; c < 3; ++c)
                 for (int o = 0; o < 3; ++o)
-                    if (o != c && (out[c] == stage[o] || out[c] == pos[o] || out[c] == tens[o] || out[c] == tensstage[o]))
+                    if (out[c] == wcon || o != c && (out[c] == stage[o] || out[c] == pos[o] || out[c] == tens[o] || out[c] == tensstage[o]))
                         apart = false;
             if (apart && tma_wanted(variant, tune)) {
                 const int arc = launch_tma<S, C>(p, stream, comps, wcon, ni, nj, nk, si, sj, sk);

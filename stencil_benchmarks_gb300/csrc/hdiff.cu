@@ -190,10 +190,12 @@ __global__ void __launch_bounds__(256)
 // for VEC j/k strides multiples of the vector size, and inp / coeff / out at
 // the same offset from a vector boundary (then one column grid is
 // vector-aligned in all three fields); SB_ERR_UNSUPPORTED (no error text) if not.
+// So is a domain too tall for the launch grid, as JSCAN's blocks cover more rows,
+// unless the caller named this variant.
 template <class S, class C, int V, bool VEC>
 int launch_vscan(const void* inp, const void* coeff, void* out, int64_t ni, int64_t nj, int64_t nk, int64_t si,
                  int64_t sj, int64_t sk, int nw, int ty, int kper, int unroll, cudaStream_t stream,
-                 const DeviceProps* p) {
+                 const DeviceProps* p, bool named = false) {
     constexpr int ES = (int)sizeof(S), VB = V * ES;
     if (si != 1 || sj <= 0 || sk <= 0) return SB_ERR_UNSUPPORTED;
     int cs0 = -2;
@@ -208,7 +210,8 @@ int launch_vscan(const void* inp, const void* coeff, void* out, int64_t ni, int6
     SB_CHECK(ty >= 1 && kper >= 1, SB_ERR_INVALID, "vscan: tile_y and k_per_cta must be positive");
     const int64_t nstrips = ceil_div(ni - (cs0 + 2), (int64_t)kStripStep<V, VEC>);
     const int64_t gx = nstrips, gy = ceil_div(ceil_div(nj, ty), (int64_t)nw), gz = ceil_div(nk, kper);
-    SB_CHECK(gy <= p->max_grid_y && gz <= p->max_grid_z, SB_ERR_INVALID, "hdiff grid too large");
+    if (gy > p->max_grid_y || gz > p->max_grid_z)
+        return named ? fail(SB_ERR_INVALID, "hdiff grid too large") : SB_ERR_UNSUPPORTED;
     const dim3 grid((unsigned)gx, (unsigned)gy, (unsigned)gz), block(32, nw);
     const int64_t lo = -(2 + V) - 2 * sj;
     const int64_t hi = ni + 2 + 32 * V + (nj + 2) * sj + nk * sk;
@@ -672,20 +675,20 @@ int launch_typed(const void* inp, const void* coeff, void* out, int64_t ni, int6
             if constexpr (sizeof(S) == 8) {
                 if (width == 64) {
                     shape_ok = true;
-                    rc2 = launch_vscan<S, C, 2, true>(inp, coeff, out, ni, nj, nk, si, sj, sk, nw, ty, kper, unroll, stream, p);
+                    rc2 = launch_vscan<S, C, 2, true>(inp, coeff, out, ni, nj, nk, si, sj, sk, nw, ty, kper, unroll, stream, p, true);
                 }
             } else if constexpr (sizeof(S) == 4) {
                 if (width == 64 || width == 128) shape_ok = true;
                 if (width == 64)
-                    rc2 = launch_vscan<S, C, 2, true>(inp, coeff, out, ni, nj, nk, si, sj, sk, nw, ty, kper, unroll, stream, p);
+                    rc2 = launch_vscan<S, C, 2, true>(inp, coeff, out, ni, nj, nk, si, sj, sk, nw, ty, kper, unroll, stream, p, true);
                 if (width == 128)
-                    rc2 = launch_vscan<S, C, 4, true>(inp, coeff, out, ni, nj, nk, si, sj, sk, nw, ty, kper, unroll, stream, p);
+                    rc2 = launch_vscan<S, C, 4, true>(inp, coeff, out, ni, nj, nk, si, sj, sk, nw, ty, kper, unroll, stream, p, true);
             } else {
                 if (width == 128 || width == 256) shape_ok = true;
                 if (width == 128)
-                    rc2 = launch_vscan<S, C, 4, true>(inp, coeff, out, ni, nj, nk, si, sj, sk, nw, ty, kper, unroll, stream, p);
+                    rc2 = launch_vscan<S, C, 4, true>(inp, coeff, out, ni, nj, nk, si, sj, sk, nw, ty, kper, unroll, stream, p, true);
                 if (width == 256)
-                    rc2 = launch_vscan<S, C, 8, true>(inp, coeff, out, ni, nj, nk, si, sj, sk, nw, ty, kper, unroll, stream, p);
+                    rc2 = launch_vscan<S, C, 8, true>(inp, coeff, out, ni, nj, nk, si, sj, sk, nw, ty, kper, unroll, stream, p, true);
             }
             SB_CHECK(shape_ok, SB_ERR_INVALID,
                      "hdiff vscan strip width (block_x) must be 64 for 8-byte, 64 or 128 for 4-byte and 128 or 256 "

@@ -596,15 +596,21 @@ int launch_typed(const void* inp, const void* coeff, void* out, int64_t ni, int6
     }
     // bfloat16 storage, float-pair and float32 compute: vector strips (V
     // columns per lane, packed float32 arithmetic) issue fewer instructions per
-    // point than JSCAN (44 vs 62 us, 273 vs 313 us and, with V = 2, 46 vs 53 us at
+    // point than JSCAN (44 vs 62 us, 267 vs 313 us and, with V = 2, 46 vs 53 us at
     // 512x512x80; 56 and 49 with scalar arithmetic and rows loaded U at a time).
     // float32 loads 8 rows at a time: 43.3 us at 512x512x80, 4 rows 46.0, 2 49.4,
     // 1 59.7 (79 and 84 us with 8 and 4 at 1024x1024x40, the same at 128x128x64);
     // the 64 registers are what that costs.  16-row tiles: 8 rows 45.4, 32 45.4.
+    // Float pairs: 8 rows where 16 leave fewer than 100 warps per SM (64x64x40 14.8
+    // us against 24.0, 128x128x64 26.9 / 31.1, 200x200x60 44.1 / 50.1, 391x263x97
+    // 140 / 147), 16 beyond (512x512x80 270 against 275 with 8).
+    auto warps_of_16_rows = [&](int64_t columns) { return ceil_div(ni, columns) * ceil_div(nj, (int64_t)16) * nk; };
+    const int pair_rows = warps_of_16_rows(60) > 100 * (int64_t)p->sm_count ? 16 : 8;
     if constexpr (std::is_same<S, bf16>::value || std::is_same<C, f32x2>::value) {
         if (variant == SB_VARIANT_AUTO) {
             constexpr int V = sizeof(S) == 8 ? 2 : 4;
-            const int rc_v = launch_vscan<S, C, V, true>(inp, coeff, out, ni, nj, nk, si, sj, sk, 1, 16, 1, 1, stream, p);
+            const int rc_v = launch_vscan<S, C, V, true>(inp, coeff, out, ni, nj, nk, si, sj, sk, 1, V == 2 ? pair_rows : 16, 1, 1,
+                                                         stream, p);
             if (rc_v != SB_ERR_UNSUPPORTED) return rc_v;
         }
     }
@@ -617,14 +623,23 @@ int launch_typed(const void* inp, const void* coeff, void* out, int64_t ni, int6
     // Rows that no aligned vectors fit (odd strides, fields at different offsets):
     // the same strips with single elements, two columns per lane; JSCAN strips
     // spend 76 instructions per point where these spend about 35.  391x263x97:
-    // bfloat16 27.0 us (JSCAN 38.2), float32 28.6 (31.1), float pair 148 (175);
-    // 1001x61x100 bfloat16 18.3 (22.2), float32 18.9 (18.9); 513x511x80 47 (60) and
-    // 51.6 (50.7).
+    // bfloat16 22.8 us (JSCAN 28.9), float32 24.8 (26.7), float pair 140 (172);
+    // 513x511x80 44.4 (57.6), 47.0 (48.5), 272 (306); 1023x1021x40 84.8 (111), 89.2
+    // (89.1), 526 (573).  float32 tiles of 8 rows where 16 leave fewer than 48 warps
+    // per SM (129x127x64 4.5 us against 5.0, 257x259x80 12.0 / 12.4), 16 beyond
+    // (513x511x80 47.0 against 49.4 with 8, 1023x1021x40 89.2 / 94.3).  Float pairs
+    // of a domain that fills the SMs stay with JSCAN where its narrower strips
+    // leave a fifth fewer lanes without a column (61x1001x100: 143 us against 148).
+    // A shape in the tune is JSCAN's.
     if constexpr (!std::is_same<C, fix64>::value && !std::is_same<C, double>::value) {
-        if (variant == SB_VARIANT_AUTO) {
+        if (variant == SB_VARIANT_AUTO && !(tune && (tune->block_x || tune->block_y || tune->tile_y || tune->k_per_cta || tune->unroll))) {
             constexpr bool f32 = std::is_same<S, float>::value, pairs = std::is_same<C, f32x2>::value;
-            const int rc_v = launch_vscan<S, C, 2, false>(inp, coeff, out, ni, nj, nk, si, sj, sk, f32 ? 2 : 1, f32 ? 8 : 16,
-                                                          1, pairs ? 1 : 4, stream, p);
+            const int64_t warps = warps_of_16_rows(60), fill = 48 * (int64_t)p->sm_count;
+            const bool idle = pairs && warps > fill && 5 * 32 * ceil_div(ni, (int64_t)kJscanOut) < 4 * 64 * ceil_div(ni, (int64_t)60);
+            const int rows = f32 ? (warps > fill ? 16 : 8) : pairs ? pair_rows : 16;
+            const int rc_v = idle ? SB_ERR_UNSUPPORTED
+                                  : launch_vscan<S, C, 2, false>(inp, coeff, out, ni, nj, nk, si, sj, sk, f32 ? 2 : 1, rows, 1,
+                                                                 pairs ? 1 : 4, stream, p);
             if (rc_v != SB_ERR_UNSUPPORTED) return rc_v;
         }
     }

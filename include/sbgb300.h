@@ -69,9 +69,10 @@ extern "C" {
                             * and float pairs, JSCAN otherwise (and for fixed64);
                             * vadv: TMEM staged by tensor copies for float32 compute
                             * (i unit-stride, 9 <= nk <= 256, no shape in the tune;
-                            * shorter columns: TMEM with staged rows from 2048 column
-                            * groups on), else SLAB / WSLAB when ccol/dcol are given,
-                            * else SMEM                                              */
+                            * fewer than 2048 column groups: nk >= 20 or ccol/dcol
+                            * given; shorter columns: TMEM with staged rows from 2048
+                            * column groups on), else SLAB / WSLAB when ccol/dcol are
+                            * given, else SMEM                                       */
 #define SB_HDIFF_TILE 1   /* smem-staged k-plane tiles, lap/flx/fly once per point */
 #define SB_HDIFF_JSCAN 2  /* register j-march, i-neighbours by warp shuffles       */
 #define SB_HDIFF_TMA 3    /* TILE with inp k-planes staged by TMA (cp.async.bulk.tensor)

@@ -712,6 +712,9 @@ TmemComponents<S> one_component(const void* stage, const void* pos, const void* 
     return comps;
 }
 
+// levels from which few column groups take the TMA-staged form (see launch_typed)
+constexpr int64_t kTmaPaysFrom = 20;
+
 // The TMA-staged form runs for AUTO without an explicit shape and for an
 // explicit TMEM variant that names neither a ring depth nor a staging form.
 bool tma_wanted(int variant, const sb_tune* tune) {
@@ -735,14 +738,20 @@ int launch_typed(const void* stage, const void* pos, const void* tens, const voi
     const size_t smem = 2 * sizeof(C) * (size_t)nk * (size_t)(bx * by);
     const bool can_global = ccol && dcol && sizeof(S) == sizeof(C);
     // float32 compute, no explicit shape: staged by TMA with factors in tensor
-    // memory at every size (figures in vadv_tma.cuh; 192 column groups of 40
-    // levels: 10.0 us on the device against 11.5 for SMEM async).  Where that
-    // form does not apply (fewer than 9 levels), row staging with factors in
-    // tensor memory from 2048 column groups of 32 on (256 x 256; below, its one
-    // block per SM is not filled), else SMEM async.
+    // memory (figures in vadv_tma.cuh; 192 column groups of 40 levels: 7.6 us on
+    // the device against 8.0 for SMEM async), but for short columns of few groups,
+    // whose time is the kernel's start and first copies: 24x24x9 4.0 us against 2.8
+    // for SMEM async, 128x128x9 4.3 / 3.2, 200x200x16 6.2 / 5.7, 128x128x17 5.5 /
+    // 4.5.  (The two meet between 24 and 32 levels; from 20 on the difference is
+    // at most 0.9 us.  With scratch fields given, the alternative would be WSLAB:
+    // 24x24x16 10.7 us against 4.9.)  Where TMA staging does not apply (fewer than 9
+    // levels), row staging with factors in tensor memory from 2048 column groups
+    // of 32 on (256 x 256; below, its one block per SM is not filled), else SMEM
+    // async.
     if constexpr (std::is_same<C, float>::value) {
         const TmemComponents<S> comps = one_component<S>(stage, pos, tens, tensstage, out, wsh);
-        if (tma_wanted(variant, tune)) {
+        const bool brief = variant == SB_VARIANT_AUTO && nk < kTmaPaysFrom && ceil_div(ni, (int64_t)32) * nj < 2048 && !(ccol && dcol);
+        if (tma_wanted(variant, tune) && !brief) {
             const int arc = launch_tma<S, C>(p, stream, comps, wcon, ni, nj, nk, si, sj, sk);
             if (arc != SB_ERR_UNSUPPORTED) return arc;
         }

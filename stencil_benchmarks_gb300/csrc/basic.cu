@@ -161,7 +161,12 @@ __global__ void __launch_bounds__(256) lap_march_kernel(const S* __restrict__ in
 // 512x512x80, an integer one 70 us of the ALU pipe.  Along x and y, of five
 // operations a point on the integer pipe: none 206 us, 1.13 163, 1.25 159, 1.38
 // 154, 1.5 154, 1.63 160, 1.75 167, 2 184 (ALU pipe 89%, fp64 56% busy); along
-// one axis 72-84 us (all fp64 87-90), along three 251 (326).
+// one axis 72-84 us (all fp64 87-90), along three 251 (326).  Few warps leave
+// both pipes idle and the integer sequences only lengthen each point's chain:
+// up to nine warps per SM all run on the fp64 pipe (along x and y / three axes, us,
+// all fp64 against the split: 64x64x20 3.5 / 4.4 against 4.5 / 6.9, 64x64x40 4.5 /
+// 6.3 against 5.1 / 7.6, 128x128x20 5.5 / 7.7 against 5.9 / 8.8; 96x96x40, 9.5
+// warps per SM, 6.2 / 8.8 against 6.1 / 8.9; 128x128x40 9.4 / 13.7 against 8.1 / 12.0).
 constexpr uint32_t kLapDefaultSites = 0x4Au;
 constexpr uint32_t lap_fewer_sites(int mask) {
     return kLapDefaultSites & ~(mask & 1 ? 0x02u : mask & 2 ? 0x08u : 0x40u);
@@ -219,7 +224,8 @@ int launch_lap_march(const void* inp, void* out, int64_t ni, int64_t nj, int64_t
              SB_ERR_INVALID, "domain too large for the Laplacian strip grid");
     const S* in = (const S*)inp;
     S* o = (S*)out;
-    const int pl = placement;
+    const int64_t strips = ceil_div(ni, (int64_t)32) * ceil_div(nj, (int64_t)rows) * ceil_div(nk, (int64_t)pk);
+    const int pl = placement == 0 && strips <= 9 * (int64_t)p->sm_count ? 1 : placement;
     switch (mask) {
 #define SB_LAP_MASK(M) \
     case M: return launch_lap_march_shape<M, S, C>(rows, pk, pl, in, o, ni, nj, nk, si, sj, sk, warps, stream);

@@ -291,8 +291,8 @@ int sb_vadv3(int storage, int compute, const void* const* stage, const void* con
  * same hdiff / vadv computations.  A batch holds up to max_domains domains of
  * one (storage, compute) form; sb_batch_launch runs all of them in one graph
  * launch (captured on the first launch) of persistent kernels -- one for the
- * hdiff domains, one for the vadv domains (float32 compute, i unit-stride, at
- * least 17 levels each) or one per nk bucket of them, running side by side
+ * hdiff domains, one for the vadv domains (float32 compute, i unit-stride, 9 to
+ * 256 levels each) or one per nk bucket of them, running side by side
  * -- that pull work items from device-side queues.  Results
  * are bit-identical to sb_hdiff / sb_vadv on the same domain.  The domain
  * table lives in pinned host memory and is copied by each launch: do not

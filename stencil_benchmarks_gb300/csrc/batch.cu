@@ -24,9 +24,9 @@
 //   frees shared memory for more blocks per SM.  Domains are grouped into 8 nk
 //   buckets (caps max_nk/8, 2*max_nk/8, ...) and each bucket's kernel and slab
 //   are sized for its cap, so short columns do not pay for the tallest one.
-//   With float32 arithmetic, i unit-stride and no column shorter than 17 levels
-//   all vadv domains run in one kernel instead, staged by TMA from one queue
-//   (batch_vadv_tma_kernel).
+//   With float32 arithmetic, i unit-stride and columns of 9 to 256 levels all
+//   vadv domains run in one kernel instead, staged by TMA from one queue
+//   (batch_vadv_tma_kernel), unless most columns are short (tma_of_set).
 // No kernel waits on another warp or kernel: every queue is one atomic counter.
 #include <algorithm>
 #include <cstring>
@@ -56,6 +56,7 @@ struct DevDomain {
     int32_t vec;  // hdiff: aligned vectors of the strip form fit this domain's rows
     int32_t cs0;  // ... first column of strip 0 then
     int32_t drift, off[kTmaFields];  // vadv by TMA (vadv_tma.cuh)
+    int32_t chunk;                   // ... column groups of an item
     CUtensorMap maps[kTmaFields];
 };
 static_assert(alignof(DevDomain) % 64 == 0, "tensor maps lie on 64-byte boundaries");
@@ -275,6 +276,7 @@ constexpr int kTmemDepth = 8;
 // each with its own last round.
 struct TmaBatch {
     int nt, stages, stage_bytes, warp_bytes, polls;
+    int chunks;  // whether items of the set have more than one column group
     int* status;
 };
 template <class S, int R>
@@ -293,16 +295,29 @@ __global__ void __launch_bounds__(512, 1)
     unsigned char* const mem = smem_tma + B::ring_offset(nwarps) + warp * a.warp_bytes;
     pipe.init(mem, smem_tma + 16 + warp * B::BAR_BYTES, lane, a.stages, a.stage_bytes, a.polls);
     float* const fmem = reinterpret_cast<float*>(mem + a.stages * a.stage_bytes + kTmaPosStages * B::POSB);
-    int known = -1;  // domain whose maps this warp has acquired last
+    int known = -1;          // domain whose maps this warp has acquired last
+    int dom = first;         // of the warp's item
+    int group = 0, end = 0;  // its column groups not taken yet (a.chunks)
     auto take = [&]() {
         TmaSolve<S> v;
         unsigned long long item = 0;
-        if (lane == 0) item = atomicAdd(counter, 1ULL);
-        item = __shfl_sync(0xffffffffu, item, 0);
-        v.live = (int64_t)item < total;
-        const int lo = v.live ? find_domain(tab, first, last - 1, (int64_t)item) : first;
+        v.live = true;
+        if (!a.chunks || group == end) {
+            if (lane == 0) item = atomicAdd(counter, 1ULL);
+            item = __shfl_sync(0xffffffffu, item, 0);
+            v.live = (int64_t)item < total;
+            if (v.live) dom = find_domain(tab, first, last - 1, (int64_t)item);
+        }
+        const int lo = dom;
         const DevDomain& dm = tab->dom[lo];
-        const int local = (int)((int64_t)item - dm.item_begin);
+        int local = (int)((int64_t)item - dm.item_begin);
+        if (a.chunks) {
+            if (group == end && v.live) {
+                group = local * dm.chunk;
+                end = min(group + dm.chunk, dm.items_i * dm.items_j);
+            }
+            local = v.live ? group++ : 0;
+        }
         const int i0 = v.live ? (local % dm.items_i) * 32 : 0, j = v.live ? local / dm.items_i : 0;
         const uintptr_t maps = (uintptr_t)dm.maps;
         v.maps = (const CUtensorMap*)((uintptr_t)(uint32_t)uniform((int)(uint32_t)(maps >> 32)) << 32 |
@@ -345,7 +360,7 @@ constexpr int kTmaClasses = 3;
 struct TmaClass {
     void (*run)(dim3, dim3, size_t, cudaStream_t, const DevTable*, unsigned long long*, const TmaBatch&);
     const void* fn;
-    TmaShape (*shape)(bool far, int64_t max_nk, int sms, int smem_optin);
+    TmaShape (*shape)(bool far, int64_t max_nk, int64_t min_nk, int64_t groups, int max_warps, int sms, int smem_optin);
     bool (*encode)(CUtensorMap*, int*, const void* const (&)[kTmaFields], int64_t, int64_t, int64_t, int64_t, int64_t,
                    int64_t);
     int (*stage_bytes)(bool far);
@@ -400,9 +415,8 @@ TmaClass tma_class() {
         batch_vadv_tma_kernel<S, R><<<g, b, smem, s>>>(t, q, a);
     };
     c.fn = (const void*)&batch_vadv_tma_kernel<S, R>;
-    // the most warps (a batch has more column groups than any launch has warps)
-    c.shape = [](bool far, int64_t max_nk, int sms, int optin) {
-        return tma_shape<S, R>(far, max_nk, (int64_t)1 << 40, sms, optin);
+    c.shape = [](bool far, int64_t max_nk, int64_t min_nk, int64_t groups, int max_warps, int sms, int optin) {
+        return tma_shape<S, R>(far, max_nk, min_nk, groups, max_warps, sms, optin);
     };
     c.encode = [](CUtensorMap* m, int* off, const void* const (&f)[kTmaFields], int64_t ni, int64_t nj, int64_t nk,
                   int64_t sj, int64_t sk, int64_t wsh) {
@@ -483,6 +497,7 @@ using namespace sb;
 
 struct sb_batch {
     int device = 0;
+    DeviceProps props{};
     int storage = 0, compute = 0;
     int max_domains = 0;
     int64_t max_nk = 0;
@@ -514,9 +529,11 @@ struct sb_batch {
     int vadv_tmem_grid = 0;
     size_t tmem_smem = 0;
     // float32 vadv staged by TMA: what the current domain set uses and what the captured graph has
-    // (drift class + kTmaClasses where a domain reads wcon at j + 1; -1: not this form)
+    // (drift class + kTmaClasses where a domain reads wcon at j + 1; -1: not this form), and the
+    // launch shapes, which the set's tallest and shortest columns give
     int use_tma = -1, graph_tma = -1;
-    TmaShape tma_shapes[2 * kTmaClasses] = {};
+    TmaShape tma_shape{}, graph_shape{};
+    bool tma_chunks = false, graph_chunks = false;
     BatchStatus status;  // its word lies behind host_table
     int graph_polls = 0;
 };
@@ -546,14 +563,36 @@ size_t vadv_smem_bytes(int cap, int bt, int cbytes, int sbytes, int depth, int* 
     return fac + (size_t)(depth + 1) * 6 * bt * sbytes;
 }
 
+// Column groups of an item of the TMA-staged queue.  Of short columns a warp takes
+// several with one look at the counter, as long as every warp gets four items
+// (24 domains of 100-400 columns a side, vadv alone: 9 to 16 levels float32 379 ->
+// 177 us, bfloat16 346 -> 158; 17 to 24 levels 262 -> 234 and 233 -> 195).  From 40
+// levels on two groups an item are slower (545 -> 641): neighbouring groups are
+// then not in flight together.
+int64_t tma_chunk(int64_t nk, int64_t groups, int64_t warps) {
+    return std::max<int64_t>(1, std::min(1536 / (nk * nk), groups / (4 * warps)));
+}
+
 // Drift class of the set's vadv domains (see sb_batch::use_tma) where the TMA
-// form takes all of them, else -1.
-int tma_of_set(const sb_batch* b, const Kinds& k, const sb_domain* domains, const std::vector<int> (&vd)[kBuckets]) {
-    if (!k.tma[0].run) return -1;
+// form takes all of them, else -1; the launch shape for them and their column
+// groups.  The shape follows the set's tallest and shortest columns.  (With that
+// of a capacity of 256 levels instead, the 64 uneven domains up to 137 take 1682 us
+// in float32 and 1387 in bfloat16, not 1320 and 1001.)
+// Warps per block (us with 16 / 8 at most): 8 beside hdiff domains, which get the
+// shared memory that they leave (24 + 24 domains of 40-80 levels, 100-400 columns a
+// side, float32 847 / 688, bfloat16 801 / 775), and for many float32 columns (6 x
+// 512x256x64 302 / 251), 16 otherwise (24 vadv domains of 20-80 levels, 40-200
+// columns a side, float32 107 / 118; bfloat16, 100-400 a side, 340 / 431).
+// Short columns alone stay with the bucket kernels (9-16 levels, 40-200 columns a
+// side, float32 59 us against 81, bfloat16 57 / 67; many float32 columns of 17-24
+// levels 222 / 228), but not few of them (four of 64x48x12: 30 us, staged by TMA 17).
+int tma_of_set(const sb_batch* b, const Kinds& k, const sb_domain* domains, const std::vector<int> (&vd)[kBuckets],
+               bool hdiff, TmaShape* shape, int64_t* groups) {
+    if (!k.tma[0].run || b->vadv_block != 32) return -1;
     const int es = storage_size(b->storage);
     int cls = 0;
     bool far = false;
-    int64_t min_nk = 1 << 30;
+    int64_t min_nk = 1 << 30, max_nk = 0, levels = 0;
     for (const auto& v : vd) {
         for (int q : v) {
             const sb_domain& s = domains[q];
@@ -566,6 +605,10 @@ int tma_of_set(const sb_batch* b, const Kinds& k, const sb_domain* domains, cons
             if (drift != 0) cls = std::max(cls, drift == 8 ? 1 : 2);
             far |= (int64_t)s.wshift_j * s.sj > 1;
             min_nk = std::min(min_nk, s.nk);
+            max_nk = std::max(max_nk, s.nk);
+            const int64_t count = ceil_div(s.ni, (int64_t)32) * s.nj;
+            *groups += count;
+            levels += count * s.nk;
         }
     }
     // one exact class for the whole set: drift 0 and 8 together are "any"
@@ -574,9 +617,16 @@ int tma_of_set(const sb_batch* b, const Kinds& k, const sb_domain* domains, cons
             for (int q : v)
                 if (domains[q].ni && domains[q].nj && domains[q].sk * es % 16 == 0) cls = 2;
     const int use = cls + (far ? kTmaClasses : 0);
-    const TmaShape& sh = b->tma_shapes[use];
-    if (sh.warps < 1 || min_nk < tma_min_levels(sh.stages)) return -1;
-    return use;
+    if (max_nk == 0) min_nk = max_nk = tma_min_levels(kTmaMaxStages);  // no columns: one kernel that returns at once
+    if (max_nk > 256) return -1;
+    const int sms = b->props.sm_count;
+    const bool many = es == 4 && *groups > 128 * (int64_t)sms;
+    if (!hdiff && *groups > 16 * (int64_t)sms && levels < *groups * (many ? 24 : 17)) return -1;
+    // no more warps than a single round of few columns takes (four domains of 64x48x12: 17 us, with 16 warps 21)
+    const int max_warps = hdiff || many ? 8 : kTmaMaxWarps;
+    const int64_t as_if = *groups <= (int64_t)sms * max_warps ? std::max<int64_t>(1, *groups) : (int64_t)1 << 40;
+    *shape = k.tma[cls].shape(far, max_nk, min_nk, as_if, max_warps, sms, b->props.smem_optin);
+    return shape->warps < 1 ? -1 : use;
 }
 
 int capture_graph(sb_batch* b) {
@@ -588,9 +638,7 @@ int capture_graph(sb_batch* b) {
         cudaGraphDestroy(b->graph);
         b->graph = nullptr;
     }
-    const DeviceProps* p;
-    const int prc = device_props(&p);
-    if (prc) return prc;
+    const DeviceProps* const p = &b->props;
     Kinds k;
     SB_CHECK(pick_kinds(b->storage, b->compute, b->idx64, &k), SB_ERR_UNSUPPORTED, "unsupported form");
     auto vadv_run = b->vadv_block == 64 ? k.vadv64 : k.vadv32;
@@ -608,8 +656,8 @@ int capture_graph(sb_batch* b) {
     size_t tma_smem = 0;
     if (b->use_tma >= 0) {
         const TmaClass& c = k.tma[b->use_tma % kTmaClasses];
-        const TmaShape& sh = b->tma_shapes[b->use_tma];
-        ta = {sh.nt, sh.stages, c.stage_bytes(b->use_tma >= kTmaClasses), sh.warp_bytes, wait_polls(), b->status.word};
+        const TmaShape& sh = b->tma_shape;
+        ta = {sh.nt, sh.stages, c.stage_bytes(b->use_tma >= kTmaClasses), sh.warp_bytes, wait_polls(), b->tma_chunks, b->status.word};
         tma_smem = std::max<size_t>(c.ring_offset(sh.warps) + (size_t)sh.warps * sh.warp_bytes, 120 * 1024);
         const int rc = allow_smem(c.fn, p);
         if (rc) return rc;
@@ -626,9 +674,9 @@ int capture_graph(sb_batch* b) {
     // order 0: hdiff first, then the vadv buckets; order 1: the vadv buckets
     // first (tallest first), so their blocks are resident before the hdiff
     // blocks take the remaining room of each SM.  The TMA form, whose one block
-    // per SM otherwise waits for that room, always goes first (64 uneven
-    // domains: float32 1321 us against 1454, bfloat16 1158 against 1532; the
-    // float64 slab buckets gain nothing from it, 980 against 832 for 8 domains).
+    // per SM otherwise waits for that room, always goes first (24 + 24 domains of
+    // 80-137 levels, 100-400 columns a side: float32 1236 us against 1412, bfloat16
+    // 1279 against 1594; the float64 slab buckets gain nothing from it).
     const bool vadv_first = b->tune.order == 1 || b->use_tma >= 0;
     auto launch_hdiff = [&]() {
         cudaStreamWaitEvent(b->streams[1], b->fork, 0);
@@ -640,7 +688,7 @@ int capture_graph(sb_batch* b) {
     for (int qq = 0; qq < nvadv; ++qq) {
         if (nvadv == 1) {
             cudaStreamWaitEvent(b->streams[2], b->fork, 0);
-            k.tma[b->use_tma % kTmaClasses].run(dim3(b->vadv_tmem_grid), dim3(32 * b->tma_shapes[b->use_tma].warps),
+            k.tma[b->use_tma % kTmaClasses].run(dim3(p->sm_count), dim3(32 * b->tma_shape.warps),
                                                 tma_smem, b->streams[2], b->dev_table, b->counters + 1, ta);
             cudaEventRecord(b->joins[1], b->streams[2]);
             break;
@@ -668,6 +716,8 @@ int capture_graph(sb_batch* b) {
     b->graph_idx64 = b->idx64;
     b->graph_tmem = b->use_tmem;
     b->graph_tma = b->use_tma;
+    b->graph_shape = b->tma_shape;
+    b->graph_chunks = b->tma_chunks;
     return SB_OK;
 }
 
@@ -691,14 +741,15 @@ int sb_batch_create(sb_batch** out, int storage, int compute, int max_domains, i
     if (rc) return rc;
     sb_batch* b = new sb_batch();
     b->device = p->device;
+    b->props = *p;
     b->storage = storage;
     b->compute = compute;
     b->max_domains = max_domains;
     b->max_nk = max_nk;
     if (tune) b->tune = *tune;
     b->hdiff_block = b->tune.block > 0 ? b->tune.block : 128;
-    // 8 blocks per SM: 64 uneven domains, half of them hdiff, float32 1419 us (the
-    // hdiff ones alone 544) against 1678 (774) with 4; bfloat16 1443 against 2062
+    // 8 blocks per SM: of 64 uneven domains the hdiff ones alone take 544 us in
+    // float32, 774 with 4 blocks
     const int per_sm = b->tune.blocks_per_sm > 0 ? b->tune.blocks_per_sm : 8;
     b->vadv_block = b->tune.vadv_block > 0 ? b->tune.vadv_block : 32;
     if (b->hdiff_block % 32 || b->hdiff_block > 256 || per_sm > 32 || (b->vadv_block != 32 && b->vadv_block != 64)) {
@@ -749,9 +800,6 @@ int sb_batch_create(sb_batch** out, int storage, int compute, int max_domains, i
         }
         b->tmem_smem = smem;
         b->vadv_tmem_grid = p->sm_count;
-        for (int q = 0; q < 2 * kTmaClasses; ++q)
-            if (k.tma[q % kTmaClasses].run && max_nk >= tma_min_levels(2))
-                b->tma_shapes[q] = k.tma[q % kTmaClasses].shape(q >= kTmaClasses, max_nk, p->sm_count, p->smem_optin);
     }
     size_t slab_total = 0;
     size_t slab_off[kBuckets] = {};
@@ -838,11 +886,13 @@ int sb_batch_set(sb_batch* b, const sb_domain* domains, int n) {
     bool tmem_ok = b->tmem_capable;
     Kinds k;
     SB_CHECK(pick_kinds(b->storage, b->compute, false, &k), SB_ERR_UNSUPPORTED, "unsupported form");
-    int tma = b->tmem_capable ? tma_of_set(b, k, domains, vd) : -1;
+    TmaShape shape{};
+    int64_t groups = 0;
+    int tma = tma_of_set(b, k, domains, vd, !hd.empty(), &shape, &groups);
     const int es = storage_size(b->storage);
     DevTable* t = b->host_table;
     int slot = 0;
-    bool encoded = true;
+    bool encoded = true, chunks = false;
     auto fill = [&](int q, int64_t& items) {
         const sb_domain& s = domains[q];
         DevDomain& d = t->dom[slot++];
@@ -890,7 +940,9 @@ int sb_batch_set(sb_batch* b, const sb_domain* domains, int n) {
             }
             d.items_i = (int32_t)ceil_div(s.ni, b->vadv_block);
             d.items_j = (int32_t)s.nj;
-            items += (int64_t)d.items_i * d.items_j;
+            d.chunk = tma >= 0 ? (int32_t)tma_chunk(s.nk, groups, b->props.sm_count * shape.warps) : 1;
+            chunks |= d.chunk > 1;
+            items += ceil_div((int64_t)d.items_i * d.items_j, (int64_t)d.chunk);
         }
     };
     int64_t total = 0;
@@ -933,6 +985,8 @@ int sb_batch_set(sb_batch* b, const sb_domain* domains, int n) {
     b->idx64 = idx64;
     b->use_tmem = tmem_ok && !idx64;
     b->use_tma = tma;
+    b->tma_shape = shape;
+    b->tma_chunks = chunks;
     return SB_OK;
 }
 
@@ -947,7 +1001,8 @@ int sb_batch_launch(sb_batch* b, void* stream, double* time_s) {
     int rc = begin_batch_launch(&b->status, (cudaStream_t)stream);
     if (rc) return rc;
     if (!b->exec || b->graph_idx64 != b->idx64 || b->graph_tmem != b->use_tmem || b->graph_tma != b->use_tma ||
-        (b->use_tma >= 0 && b->graph_polls != wait_polls())) {
+        (b->use_tma >= 0 && (b->graph_polls != wait_polls() || !(b->graph_shape == b->tma_shape) ||
+                             b->graph_chunks != b->tma_chunks))) {
         rc = capture_graph(b);
         if (rc) return rc;
     }

@@ -626,7 +626,7 @@ int launch_tma_maps(const DeviceProps* p, cudaStream_t stream, const TmemCompone
     a.drift = (int)(sk * (int64_t)sizeof(S) % 16);
     a.stage_bytes = B::stage_bytes(far);
     const int64_t ngroups = ceil_div(ni, (int64_t)32) * nj;
-    const TmaShape shape = tma_shape<S, R>(far, nk, ngroups, p->sm_count, p->smem_optin);
+    const TmaShape shape = tma_shape<S, R>(far, nk, nk, ngroups, kTmaMaxWarps, p->sm_count, p->smem_optin);
     if (shape.warps < 1) return SB_ERR_UNSUPPORTED;
     a.stages = shape.stages;
     a.nt = shape.nt;

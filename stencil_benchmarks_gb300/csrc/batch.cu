@@ -760,6 +760,7 @@ int sb_batch_create(sb_batch** out, int storage, int compute, int max_domains, i
     if (b->tune.hdiff_rows <= 0) b->tune.hdiff_rows = 32;
     if (b->tune.hdiff_planes <= 0) b->tune.hdiff_planes = 1;
     b->hdiff_grid = p->sm_count * per_sm;
+    if (k.sift) b->hdiff_block = 32 * kSiftWarps;
     if (k.sift && b->tune.blocks_per_sm <= 0) b->hdiff_grid = p->sm_count * 12;
     for (int q = 0; q < kBuckets; ++q) {
         b->cap[q] = (int)std::max<int64_t>(2, ceil_div(max_nk * (q + 1), kBuckets));

@@ -479,7 +479,8 @@ extern "C" {
 
 const char* sb_last_error(void) { return g_error.c_str(); }
 
-int sb_version(void) { return 10000; }
+// raised with every change of the kernels that can change which launch shape is the fastest
+int sb_version(void) { return 10100; }
 
 int sb_device_count(int* count) {
     SB_CHECK(count, SB_ERR_INVALID, "count is NULL");

@@ -56,3 +56,8 @@ def test_a_captured_graph_follows_the_set(lib):
     for sizes in ([(34, 6, 256)], [(34, 6, 9), (62, 30, 12)], [(34, 6, 80), (33, 8, 17)], [(33, 12000, 10), (30, 9, 64)],
                   [(34, 6, 256), (34, 6, 9)], [(34, 6, 5)], [(34, 6, 256)]):
         _run(batch, [_domain("vadv", size, "float32", 7) for size in sizes], f"set {sizes}")
+
+
+def test_info_reports_the_block_that_runs(lib):
+    assert Batch("float64", block=256).info()["block"] == 128  # exact float64 has one block size
+    assert Batch("float32", block=256).info()["block"] == 256

@@ -25,6 +25,29 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA GPU and the built libsbgb300.so")
 
 
+# Modules that import the host framework (the reference's package) while they are
+# collected: without a copy of it they are skipped with the reason, as their
+# import would end the whole run.
+HOST_MODULES = {"test_collection.py", "test_gpu_benchmarks.py"}
+
+
+class _HostModule(pytest.Module):
+    def collect(self):
+        from stencil_benchmarks_gb300 import host
+
+        try:
+            host.load()
+        except host.HostFrameworkMissing as err:
+            pytest.skip(str(err), allow_module_level=True)
+        return super().collect()
+
+
+def pytest_pycollect_makemodule(module_path, parent):
+    if module_path.name in HOST_MODULES:
+        return _HostModule.from_parent(parent, path=module_path)
+    return None
+
+
 def golden_cases():
     return json.loads((GOLDEN / "cases.json").read_text())
 

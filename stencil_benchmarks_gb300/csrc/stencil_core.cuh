@@ -1062,11 +1062,11 @@ __device__ __forceinline__ void vadv_warp_column(const S* __restrict__ stage, co
 // pos rows are staged for the backward sweep.  `tcol` is the TMEM address
 // of lane 0 / column 0 of this warp's range (lane field 32 * (warp % 4)); the
 // range holds 2 * ceil(nk / 8) * 8 columns.  All 32 lanes must call this.
-// All 512 columns for the block (every warp calls it; warp 0 allocates through
-// the shared word s_taddr), and their release after the last use.
-__device__ __forceinline__ uint32_t tmem_alloc_all(uint32_t* s_taddr, int warp) {
+// `ncols` columns for the block (32, 64 .. 512; every warp calls it; warp 0 allocates
+// through the shared word s_taddr), and their release after the last use.
+__device__ __forceinline__ uint32_t tmem_alloc_all(uint32_t* s_taddr, int warp, uint32_t ncols = 512u) {
     if (warp == 0) {
-        const uint32_t dst = (uint32_t)__cvta_generic_to_shared(s_taddr), ncols = 512u;
+        const uint32_t dst = (uint32_t)__cvta_generic_to_shared(s_taddr);
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(dst), "r"(ncols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
@@ -1076,14 +1076,12 @@ __device__ __forceinline__ uint32_t tmem_alloc_all(uint32_t* s_taddr, int warp) 
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     return *reinterpret_cast<volatile uint32_t*>(s_taddr);
 }
-__device__ __forceinline__ void tmem_free_all(uint32_t tbase, int warp) {
+__device__ __forceinline__ void tmem_free_all(uint32_t tbase, int warp, uint32_t ncols = 512u) {
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    if (warp == 0) {
-        const uint32_t ncols = 512u;
+    if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tbase), "r"(ncols) : "memory");
-    }
 }
 __device__ __forceinline__ void tmem_st2(uint32_t taddr, float a, float b) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1, %2};\n" ::"r"(taddr), "r"(__float_as_uint(a)),

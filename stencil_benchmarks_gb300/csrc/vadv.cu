@@ -542,11 +542,13 @@ struct TmaArgs {
     S* out[NC];
     int off[NC][kTmaFields];
     int wsh[NC];
-    int ni, nj, nk, sj, sk, drift, nt, polls, stages, stage_bytes, warp_bytes;
+    int ni, nj, nk, sj, sk, drift, nt, polls, stages, stage_bytes, warp_bytes, tmem_cols;
     int* status;
 };
 
-template <class S, int R, int NC>
+// ALL: the block takes every column of tensor memory (a template parameter, as the
+// run-time count alone made the bfloat16 kernel of odd level strides 2% slower).
+template <class S, int R, int NC, bool ALL>
 __global__ void __launch_bounds__(512, 1) vadv_tma_kernel(const __grid_constant__ TmaArgs<S, NC> a) {
     extern __shared__ __align__(128) unsigned char smem_tma[];
     using B = TmaBox<S, R>;
@@ -554,7 +556,7 @@ __global__ void __launch_bounds__(512, 1) vadv_tma_kernel(const __grid_constant_
     const int warp = uniform((int)(threadIdx.x >> 5)), lane = threadIdx.x & 31;
     const int nwarps = blockDim.x >> 5;
     uint32_t* s_taddr = reinterpret_cast<uint32_t*>(smem_tma);
-    const uint32_t tbase = tmem_alloc_all(s_taddr, warp);
+    const uint32_t tbase = tmem_alloc_all(s_taddr, warp, ALL ? 512u : (uint32_t)a.tmem_cols);
     const uint32_t tcol = tbase + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)((warp >> 2) * a.nt * kTmaBlockCols);
     TmaPipe<S, R> pipe;
     unsigned char* const mem = smem_tma + B::ring_offset(nwarps) + warp * a.warp_bytes;
@@ -598,7 +600,7 @@ __global__ void __launch_bounds__(512, 1) vadv_tma_kernel(const __grid_constant_
             break;
         cur = next;
     }
-    tmem_free_all(tbase, warp);
+    tmem_free_all(tbase, warp, ALL ? 512u : (uint32_t)a.tmem_cols);
 }
 
 template <class S, int R, int NC>
@@ -631,15 +633,23 @@ int launch_tma_maps(const DeviceProps* p, cudaStream_t stream, const TmemCompone
     a.stages = shape.stages;
     a.nt = shape.nt;
     a.warp_bytes = shape.warp_bytes;
-    // at least 120 KB: one block per SM, so the 512-column allocation is free
-    const size_t smem = std::max<size_t>(B::ring_offset(shape.warps) + (size_t)shape.warps * shape.warp_bytes, 120 * 1024);
+    // Columns for the block's factors alone, and as much of an SM's 228 KB of shared
+    // memory as of its 512 columns, so that an allocation never waits for another
+    // block of this kernel: small launches on several streams share the SMs (eight of
+    // 64x64x40 float32 on four streams, us each: 2.4; with all columns and 120 KB for
+    // every block 5.8, on one stream 7.7 either way).
+    a.tmem_cols = 32;
+    while (a.tmem_cols < shape.nt * kTmaBlockCols * (int)ceil_div(shape.warps, 4)) a.tmem_cols *= 2;
+    const size_t share = 228 * 1024 / (512 / a.tmem_cols + 1) + 1;
+    const size_t smem = std::max<size_t>(B::ring_offset(shape.warps) + (size_t)shape.warps * shape.warp_bytes, share);
     if (status_word(stream, &a.status)) {
         clear_error();
         return SB_ERR_UNSUPPORTED;  // the forms without waits need no word
     }
-    auto kernel = vadv_tma_kernel<S, R, NC>;
-    const int rc = allow_smem<vadv_tma_kernel<S, R, NC>>(p);
+    const bool all = a.tmem_cols == 512;
+    const int rc = all ? allow_smem<vadv_tma_kernel<S, R, NC, true>>(p) : allow_smem<vadv_tma_kernel<S, R, NC, false>>(p);
     if (rc) return rc;
+    auto kernel = all ? vadv_tma_kernel<S, R, NC, true> : vadv_tma_kernel<S, R, NC, false>;
     const int64_t grid = std::min<int64_t>(p->sm_count, ceil_div(ngroups, (int64_t)shape.warps));
     t_waits = true;
     kernel<<<(unsigned)grid, (unsigned)(32 * shape.warps), smem, stream>>>(a);

@@ -435,7 +435,7 @@ template <>
 __device__ __forceinline__ f32x2 cvt<f32x2, f32x2>(f32x2 v) { return v; }
 
 // V consecutive storage elements moved as one aligned vector of V*sizeof(S)
-// bytes (4, 8 or 16), converted to / rounded from compute type C per element.
+// bytes (4, 8 or 16); st_vec rounds them from compute type C.
 template <int B>
 struct RawVec;
 template <>
@@ -450,16 +450,6 @@ template <>
 struct RawVec<16> {
     using T = uint4;
 };
-
-template <class S, class C, int V>
-__device__ __forceinline__ void ld_vec(const S* p, C (&o)[V]) {
-    using R = typename RawVec<(int)sizeof(S) * V>::T;
-    const R r = __ldg(reinterpret_cast<const R*>(p));
-    S e[V];
-    memcpy(e, &r, sizeof(R));
-#pragma unroll
-    for (int q = 0; q < V; ++q) o[q] = cvt<C, S>(e[q]);
-}
 
 template <class S, class C, int V>
 __device__ __forceinline__ void st_vec(S* p, const C (&v)[V]) {

@@ -312,7 +312,9 @@ class Server:
 
     def step(self, now: Optional[float] = None) -> bool:
         """One poll / admit / dispatch; True while requests are waiting, queued
-        or on the device."""
+        or on the device.  ``SbError`` with ``SB_ERR_TIMEOUT``: a kernel gave up
+        a bounded wait; none of the requests launched with it is completed, and
+        the next step launches them again."""
         self._check("sb_server_step", self._lib.sb_server_step(self._handle, ctypes.c_double(
             time.perf_counter() if now is None else now), ctypes.byref(self._busy)))
         self._collect()
